@@ -18,6 +18,7 @@
 
 #include "engine.hpp"
 #include "handle.hpp"
+#include "jump.hpp"
 #include "mpview.hpp"
 
 using nmg::Dbl2;
@@ -191,6 +192,7 @@ int do_upload(nm_handle* h) {
       if ((rc = upload(h->d_b32, h->b32, h->stream))) return rc;
       if ((rc = upload(h->d_c32, h->c32, h->stream))) return rc;
       if ((rc = upload(h->d_sa_min32, h->sa_min32, h->stream))) return rc;
+      if ((rc = upload(h->d_jump, h->jump, h->stream))) return rc;
     }
     if (!h->od.sa_fp64_ok) {
       if ((rc = upload(h->d_a_fe, h->od.a_fe, h->stream))) return rc;
@@ -279,6 +281,37 @@ void build_front32_tables(nm_handle* h, bool series = true) {
   }
 }
 
+// The FP32 path's jumps (jump.hpp), for |eps| up to the farthest sample's.
+void build_jump_tables(nm_handle* h, int threads) {
+  double mx = 0.0, my = 0.0;
+  int e = 0;
+  if (h->od.sa_fp64_ok) {
+    for (double x : h->eps_re) mx = std::max(mx, std::fabs(x));
+    for (double y : h->eps_im) my = std::max(my, std::fabs(y));
+  } else {
+    // every component at the largest exponent
+    e = -(1 << 30);
+    for (const nmg::RFE& x : h->eps_re_fe)
+      if (x.m != 0.0) e = std::max(e, x.e + std::ilogb(x.m));
+    for (const nmg::RFE& y : h->eps_im_fe)
+      if (y.m != 0.0) e = std::max(e, y.e + std::ilogb(y.m));
+    for (const nmg::RFE& x : h->eps_re_fe) mx = std::max(mx, std::fabs(std::scalbn(x.m, x.e - e)));
+    for (const nmg::RFE& y : h->eps_im_fe) my = std::max(my, std::fabs(std::scalbn(y.m, y.e - e)));
+  }
+  const double m = std::sqrt(mx * mx + my * my) * (1.0 + 0x1p-40);
+  nmg::build_start_jumps(h->od, m, e, threads, h->jump);
+  std::vector<nmg::JumpRec> re;
+  nmg::build_rebase_jumps(h->od, m, e, re);
+  nmg::JumpRec none{};
+  none.rho2 = -1.0f;
+  re.resize(nmg::kRebaseClasses, none);
+  // a rebase may jump when x = w^2 + (1 + Gamma) eps lies in a class in use
+  h->jump_w2 = 0.0f;
+  for (int i = 0; i < nmg::kRebaseClasses && h->jump_w2 == 0.0f; i++)
+    if (re[i].rho2 > 0.0f) h->jump_w2 = (float)std::exp2(-0.5 * nmg::kRebaseTop - i);
+  h->jump.insert(h->jump.end(), re.begin(), re.end());
+}
+
 int check_handle(const nm_handle* h) {
   if (!h) return fail(NM_ERR_ARG, "null handle");
   return NM_OK;
@@ -295,6 +328,8 @@ void set_fe_tables(const nm_handle* h, nmg::DeviceView& v) {
     v.sa_b32 = t->d_b32.p;
     v.sa_c32 = t->d_c32.p;
     v.sa_min32 = t->d_sa_min32.p;
+    v.jump = t->jump.empty() ? nullptr : t->d_jump.p;
+    v.jump_w2 = t->jump_w2;
   }
   v.sa_fe = h->od.sa_fp64_ok ? 0 : 1;
   if (!v.sa_fe) return;
@@ -443,6 +478,8 @@ nm_handle* nm_copy(const nm_handle* src) {
   h->b32 = src->b32;
   h->c32 = src->c32;
   h->sa_min32 = src->sa_min32;
+  h->jump = src->jump;
+  h->jump_w2 = src->jump_w2;
   h->reference_mode = src->reference_mode;
   h->fe_single_pass = src->fe_single_pass;
   h->fe_overlap = src->fe_overlap;
@@ -708,6 +745,7 @@ int nm_precompute(nm_handle* h) {
     h->view.eps_tables(h->od, h->eps_re, h->eps_im);
     if (!h->od.sa_fp64_ok) h->view.eps_tables_fe(h->eps_re_fe, h->eps_im_fe);
     build_front32_tables(h);
+    build_jump_tables(h, threads);
     h->precomputed = true;
   }
   h->precompute_us =

@@ -254,6 +254,64 @@ __device__ __forceinline__ TFE tfe_norm(float m, int e) {
   return TFE{ldexpf(m, -k), e + k};
 }
 
+// The polynomial of a jump's record at x (in its units), without the eps part,
+// times 2^-s: the first kJumpExact terms in float-float, the rest in FP32 (a
+// term's size falls by 2^-3 or more a degree, so their rounding is below the
+// float-float terms').
+__device__ __forceinline__ void jump_poly(const JumpRec& rec, FF xr, FF xi, FF& dr, FF& di) {
+  constexpr int n = kJumpDegree - kJumpExact;
+  float hr = rec.c[n - 1].x, hi = rec.c[n - 1].y;
+#pragma unroll
+  for (int k = n - 2; k >= 0; k--) {
+    const Flt2 c = rec.c[k];
+    const float t = fmaf(hr, xr.h, fmaf(-hi, xi.h, c.x));
+    hi = fmaf(hr, xi.h, fmaf(hi, xr.h, c.y));
+    hr = t;
+  }
+  FF pr{hr, 0.0f}, pi{hi, 0.0f};
+#pragma unroll 1
+  for (int k = kJumpExact - 1; k >= 0; k--) {
+    const Flt4 b = rec.b[k];
+    FF nr, ni;
+    ff_cmul_add(pr, pi, xr, xi, FF{b.x, b.y}, FF{b.z, b.w}, nr, ni);
+    pr = nr;
+    pi = ni;
+  }
+  ff_cmul_add(pr, pi, xr, xi, FF{0.0f, 0.0f}, FF{0.0f, 0.0f}, dr, di);
+}
+
+// The jump (jump.hpp) of a sample that stops the series at `fire`: its delta at
+// the jump's index `found`, within `dbound`; false when it has none.
+// Bit-for-bit the same start in every kernel.
+__device__ __forceinline__ bool fe_jump(const DeviceView& v, int fire, const FFE& er,
+                                        const FFE& ei, CFF& d, float& dbound, int& found) {
+  if (!v.jump) return false;
+  const JumpRec* rec = v.jump;
+  int c = 0;
+  for (; c < kJumpClasses; c++, rec += kJumpSubs) {
+    if (rec->fire == fire) break;
+    if (rec->fire < 0) return false;
+  }
+  if (c == kJumpClasses) return false;
+  // the smallest radius that holds the sample
+  const JumpRec* use = nullptr;
+  FF xr{0.0f, 0.0f}, xi{0.0f, 0.0f};
+  for (int k = kJumpSubs - 1; k >= 0 && !use; k--) {
+    if (!(rec[k].rho2 > 0.0f) || max(er.e, ei.e) - rec[k].p > 20) continue;
+    xr = ffe_scaled(er.h, er.l, er.e - rec[k].p);
+    xi = ffe_scaled(ei.h, ei.l, ei.e - rec[k].p);
+    if (fmaf(xr.h, xr.h, xi.h * xi.h) <= rec[k].rho2) use = rec + k;
+  }
+  // (an x whose square vanishes would lose its own low bits: 2^-40 and below
+  // starts at the series stop)
+  if (!use || fmaxf(fabsf(xr.h), fabsf(xi.h)) < 0x1p-40f) return false;
+  jump_poly(*use, xr, xi, d.re, d.im);
+  d.e = use->s;
+  dbound = use->err;
+  found = use->n;
+  return true;
+}
+
 __device__ __forceinline__ int fe_front32(const DeviceView& v, int r, int c, FeState& st) {
   if (v.cardioid_mode == CARDIOID_PER_SAMPLE || !v.sa_min32) return kFront32Undecided;
   const FFE er = v.eps32_re[c], ei = v.eps32_im[r];
@@ -272,12 +330,14 @@ __device__ __forceinline__ int fe_front32(const DeviceView& v, int r, int c, FeS
       fire = i1;
     }
   }
-  const int dsize = fire < n ? (fire - 3 < 1 ? 1 : fire - 3) : n;
-  const int found = dsize - 1;
+  int dsize = fire < n ? (fire - 3 < 1 ? 1 : fire - 3) : n;
+  int found = dsize - 1;
   // d[found] and its distance bound, both at exponent de
   CFF d;
   float dbound;  // in units of 2^d.e
-  if (found == 0) {
+  if (fe_jump(v, fire, er, ei, d, dbound, found)) {
+    dsize = found + 1;
+  } else if (found == 0) {
     d = eps;
     dbound = up_mul(0x1p-46f, cff_l1(eps));
   } else {
@@ -423,6 +483,105 @@ __device__ __forceinline__ void fe_renormalise(FeState& st) {
     st.err = ldexpf(st.err, st.E);
     st.E = 0;
   }
+}
+
+// The jump (jump.hpp) of a sample that has just rebased (j = 0, delta = Y = w):
+// its next n + 1 steps at once, where w^2 + (1 + Gamma) eps lies in the ball of
+// a record.  The bound passes through the jump by the polynomial's derivative
+// bound: e' = 2|w| e + e^2 + rounding of x, e'' = lip e' + err.
+__device__ __forceinline__ void fe_rebase_jump(const DeviceView& v, FeState& st) {
+  const float wl1 = up_add(fabsf(st.dr.h), fabsf(st.di.h));
+  if (!(fmaf(st.dr.h, st.dr.h, st.di.h * st.di.h) < v.jump_w2)) return;
+  // class i: |x|^2 < 2^-(kRebaseTop + 2 i), i from the exponent of |w^2 + eps|^2
+  const float ar = fmaf(st.dr.h, st.dr.h, fmaf(-st.di.h, st.di.h, st.er.h));
+  const float ai = fmaf(2.0f * st.dr.h, st.di.h, st.ei.h);
+  int i = (126 - kRebaseTop - (__float_as_int(fmaf(ar, ar, ai * ai)) >> 23)) >> 1;
+  const JumpRec* base = v.jump + kJumpClasses * kJumpSubs;
+  const FF zero{0.0f, 0.0f};
+  const JumpRec* use = nullptr;
+  FF sr = zero, si = zero;
+  // its own class, or up to two larger ones (below the smallest class its bound
+  // would be far above delta's own scale)
+  for (int t = 0; t < 3 && !use; t++, i--) {
+    if (i < 0) return;
+    if (i >= kRebaseClasses || !(base[i].rho2 > 0.0f)) continue;
+    // x = w^2 + (1 + Gamma) eps, in the record's units
+    const Flt4 g = base[i].gamma;
+    FF gr, gi, xr, xi;
+    ff_cmul_add(st.er, st.ei, FF{g.x, g.y}, FF{g.z, g.w}, zero, zero, gr, gi);
+    ff_cmul_add(st.dr, st.di, st.dr, st.di, gr, gi, xr, xi);
+    sr = ff_scale(xr, -base[i].p);
+    si = ff_scale(xi, -base[i].p);
+    if (fmaf(sr.h, sr.h, si.h * si.h) <= base[i].rho2) use = base + i;
+  }
+  if (!use) return;
+  const int n = use->n, p = use->p, s = use->s;
+  if (st.i + n + 1 >= v.N) return;
+  // bound of x: 2 |w| e + e^2 and the products' rounding (|w| as in a step, to
+  // 2^-20 of it: a looser norm would compound over a sample's jumps)
+  const float el1 = up_add(fabsf(st.er.h), fabsf(st.ei.h));
+  const float gl1 = up_add(fabsf(use->gamma.x), fabsf(use->gamma.z));
+  const float wn = up_fma(0x1p-20f, wl1, approx_norm(st.dr.h, st.di.h));
+  float ex = up_fma(up_fma(2.0f, wn, st.err), st.err, up_mul(kFeU, up_mul(wl1, wl1)));
+  ex = up_fma(up_mul(4.0f * kFeU, gl1), el1, ex);
+  ex = up_add(ldexpf(ex, -p), 0x1p-100f);
+  if (!(ex < 0x1p-12f)) return;
+  FF dr, di;
+  jump_poly(*use, sr, si, dr, di);
+  // the orders of eps, and |d delta / dx| at x, in FP32
+  const float xh = sr.h, yh = si.h;
+  auto horner = [&](const Flt2* c, int m, float& pr, float& pi) {
+    pr = c[m - 1].x;
+    pi = c[m - 1].y;
+    for (int k = m - 2; k >= 0; k--) {
+      const float t = fmaf(pr, xh, fmaf(-pi, yh, c[k].x));
+      pi = fmaf(pr, yh, fmaf(pi, xh, c[k].y));
+      pr = t;
+    }
+  };
+  const float er = st.er.h * 0x1p32f, ei = st.ei.h * 0x1p32f;
+  if (fabsf(er) + fabsf(ei) > 0x1p-78f) {
+    float qr, qi, tr, ti;
+    auto times_eps = [&]() {
+      const float t = fmaf(qr, er, -qi * ei);
+      qi = fmaf(qr, ei, qi * er);
+      qr = t;
+    };
+    horner(use->q4, kJumpEps4, qr, qi);
+    times_eps();
+    horner(use->q3, kJumpEps3, tr, ti);
+    qr += tr;
+    qi += ti;
+    times_eps();
+    horner(use->q2, kJumpEps2, tr, ti);
+    qr += tr;
+    qi += ti;
+    times_eps();
+    horner(use->q1, kJumpEps1, tr, ti);
+    qr += tr;
+    qi += ti;
+    times_eps();
+    dr = ff_add(dr, FF{qr, 0.0f});
+    di = ff_add(di, FF{qi, 0.0f});
+  }
+  float gr = 0.0f, gi = 0.0f;
+#pragma unroll
+  for (int k = kJumpDegree; k >= 1; k--) {
+    const float cr = k > kJumpExact ? use->c[k - kJumpExact - 1].x : use->b[k - 1].x;
+    const float ci = k > kJumpExact ? use->c[k - kJumpExact - 1].y : use->b[k - 1].z;
+    const float t = fmaf(gr, xh, fmaf(-gi, yh, (float)k * cr));
+    gi = fmaf(gr, yh, fmaf(gi, xh, (float)k * ci));
+    gr = t;
+  }
+  // FP32 rounding of it (at most 2^-18 of the sum of its terms) and the second
+  // derivative over the ball of radius ex
+  const float amp = up_fma(use->lip2, ex, up_fma(0x1p-17f, use->lip, approx_norm(gr, gi)));
+  const float err = up_fma(amp, ex, use->err);
+  st.dr = ff_scale(dr, s);
+  st.di = ff_scale(di, s);
+  st.err = up_add(ldexpf(err, s), 0x1p-120f);
+  st.j = n + 1;
+  st.i += n + 1;
 }
 
 // Steps while delta is scaled: Y = Z to working precision, so the events are
@@ -636,7 +795,12 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
       }
     }
     const float d2 = fmaf(dr.h, dr.h, di.h * di.h);
-    if (r2 < d2 || j == zlast) {  // rebase to Z[0]: delta = Y in float-float
+    // A rebase is open at any step (delta = Y against Z[0] is the same point,
+    // its rounding in the bound); taken early, up to |Y| = 4 |delta|, where Y
+    // is small enough to jump from: the orbit's own near returns to 0 then end
+    // in a rebase for every sample.
+    const bool small = !kDl && r2 < v.jump_w2;
+    if (r2 < (small ? 16.0f * d2 : d2) || j == zlast) {  // rebase to Z[0]: delta = Y in float-float
       const float yerr_fe = y_err();
       const FF nyr = ff_add(FF{z.hx, z.lx}, dr);
       const FF nyi = ff_add(FF{z.hy, z.ly}, di);
@@ -647,6 +811,10 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
       z = fe_load_z<kStaged>(v, 0);
       ym = approx_norm(dr.h, di.h);
       rebases++;
+      if (small) {  // jumps with the other lanes' at the next chunk's start
+        i++;
+        break;
+      }
     }
   }
   if (kDl && trap && !done && certified && i < v.N) {
@@ -713,6 +881,7 @@ __device__ __forceinline__ bool fe_advance(const DeviceView& v, FeState& st, int
     }
     return fe_scaled_steps<kStaged, kRawT>(v, st, steps, res, executed, rebases);
   }
+  if (!v.double_loop && st.j == 0) fe_rebase_jump(v, st);
   if (v.double_loop)
     return fe_unscaled_steps<true, kStaged, kRawT>(v, st, steps, res, executed, rebases, trap);
   return fe_unscaled_steps<false, kStaged, kRawT>(v, st, steps, res, executed, rebases, nullptr);

@@ -113,9 +113,12 @@ struct nm_handle {
   std::vector<nmg::FFE> eps32_re, eps32_im;
   std::vector<nmg::CFFE> a32, b32, c32;
   std::vector<nmg::TFE> sa_min32;
+  std::vector<nmg::JumpRec> jump;
+  float jump_w2 = 0.0f;
   DevBuf<nmg::FFE> d_eps32_re, d_eps32_im;
   DevBuf<nmg::CFFE> d_a32, d_b32, d_c32;
   DevBuf<nmg::TFE> d_sa_min32;
+  DevBuf<nmg::JumpRec> d_jump;
   int reference_mode = nmg::REFERENCE_PROBES;
   // FE32 iteration pass: orbit entries staged in shared memory by the TMA unit
   // (orbit_stage.cuh), and a persisting L2 access-policy window on the orbit

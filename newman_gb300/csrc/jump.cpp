@@ -1,0 +1,623 @@
+// The polynomials of jump.hpp, on the host in double.
+#if defined(__GNUC__)
+#pragma GCC optimize("O3")
+#endif
+#include "jump.hpp"
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <thread>
+
+namespace nmg {
+
+namespace {
+
+constexpr int D = kJumpDegree;
+// Orders of eps (rebase jumps) and the terms x^0 .. of each: order 0 has x^1 ..
+// x^D, the others what FP32 holds of them (JumpRec).
+constexpr int B = kJumpOrders;
+constexpr int kTerms[B] = {D + 1, kJumpEps1, kJumpEps2, kJumpEps3, kJumpEps4};
+// R stays below 2^-46 of the linear term: half the FP32 path's rounding of one
+// step, and since R grows by 2^D an octave of delta, a tighter or looser limit
+// moves the target by a few steps only.
+constexpr double kTail = 0x1p-46;
+// A record is worth its evaluation (seven float-float multiply-adds and two
+// dozen plain ones, four steps' work, and a lane's wait for its warp) from here on.
+constexpr int kMinSteps = 16;
+
+// A rebase jump goes at most this far.
+constexpr int kRebaseReach = 4096;
+
+double norm(double re, double im) { return std::sqrt(re * re + im * im); }
+
+// 2^e as a double, 0 below the range.
+double pow2(int e) { return e < -1022 ? 0.0 : std::ldexp(1.0, std::min(e, 1023)); }
+
+// The same for n radii at once.
+void sums_pow(const double* a, int lo, int hi, const double* rho, int n, double* out) {
+  for (int i = 0; i < n; i++) out[i] = 0.0;
+  for (int k = hi; k >= lo; k--)
+    for (int i = 0; i < n; i++) out[i] = out[i] * rho[i] + a[k];
+  for (int k = 0; k < lo; k++)
+    for (int i = 0; i < n; i++) out[i] *= rho[i];
+}
+
+// Coefficients of eps^b x^k, times 2^s, for orders b < NB.
+template <int NB>
+struct Poly {
+  double re[NB][D + 1], im[NB][D + 1];
+  int s;
+};
+
+// sum_k a[k] rho^k over [lo, hi].
+double sum_pow(const double* a, int lo, int hi, double rho) {
+  double s = 0.0;
+  for (int k = hi; k >= lo; k--) s = s * rho + a[k];
+  for (int k = 0; k < lo; k++) s *= rho;
+  return s;
+}
+
+// The record of polynomial u (index n) for |x| <= rho 2^p, its bound q on
+// everything but the device's evaluation; eps: the largest |eps|.
+template <int NB>
+bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q, double eps,
+                 JumpRec& r) {
+  // x in units of 2^pr with rho in (1/2, 1], the linear coefficient in [1, 2)
+  int sh = std::ilogb(rho) + 1;
+  if (std::ldexp(rho, -sh) == 0.5) sh--;
+  const double rr = std::ldexp(rho, -sh);
+  const int k0 = std::ilogb(norm(u.re[0][1], u.im[0][1])) + sh;
+  double mag[D + 1] = {}, err = 0.0, lip = 0.0, rk = 1.0;
+  JumpRec o{};
+  double lip2 = 0.0;
+  for (int k = 1; k <= D; k++) {
+    const double re = std::ldexp(u.re[0][k], sh * k - k0);
+    const double im = std::ldexp(u.im[0][k], sh * k - k0);
+    const double m = norm(re, im);
+    lip += k * m * rk;
+    if (k > 1) lip2 += 0.5 * k * (k - 1) * m * rk / rr;
+    rk *= rr;
+    if (!(m < 0x1p100)) return false;
+    if (m < 0x1p-100) {  // far below the bound's own terms
+      err += m * rk;
+      continue;
+    }
+    mag[k] = m;
+    if (k <= kJumpExact) {
+      Flt4& b = o.b[k - 1];
+      b.x = (float)re;
+      b.y = (float)(re - (double)b.x);
+      b.z = (float)im;
+      b.w = (float)(im - (double)b.z);
+    } else {
+      // plain FP32: coefficient, operand and each of the at most 2 D roundings
+      // of the Horner chain within 2^-24 of at most twice the terms' sum
+      o.c[k - kJumpExact - 1] = {(float)re, (float)im};
+      err += 0x1p-18 * m * rk;
+    }
+  }
+  // the orders of eps in plain FP32, coefficients times 2^-32b for (2^32 eps)^b
+  Flt2* const tab[B] = {nullptr, o.q1, o.q2, o.q3, o.q4};
+  for (int b = 1; b < NB; b++) {
+    rk = std::pow(std::ldexp(eps, 32), b);
+    for (int k = 0; k < kTerms[b]; k++) {
+      const int e = sh * k - k0 - 32 * b;
+      const double re = std::ldexp(u.re[b][k], e), im = std::ldexp(u.im[b][k], e);
+      const double m = norm(re, im);
+      if (!(m < 0x1p100)) return false;
+      tab[b][k] = {(float)re, (float)im};
+      err += (0x1p-18 * m + 0x1p-100) * rk;
+      rk *= rr;
+    }
+  }
+  // Horner in float-float: p_k = p_{k+1} x + b_k rounds by at most
+  // u (|p_{k+1}|_1 |x|_1 + |b_k|_1) <= 2 u m_k with m_k = |b_k| + rho m_{k+1}
+  // (u = 1.125 * 2^-43, fe_core.cuh), then is multiplied by x k times; x (its
+  // last operation included) and b_k are float-float to 2^-45 of themselves
+  const double uu = 0x1.2p-43;
+  double m = 0.0;
+  for (int k = D; k >= 1; k--) {
+    m = mag[k] + rr * m;
+    rk = std::pow(rr, k);
+    if (k <= kJumpExact) err += 2.0 * uu * m * rk;
+    err += 0x1p-44 * k * mag[k] * rk;
+  }
+  err += 2.0 * uu * m * rr;
+  err = 1.01 * (err + std::ldexp(q, -k0));
+  // (a bound above a thousand FP32 steps' rounding is not worth the jump)
+  if (!(err < 0x1p-31)) return false;
+  o.fire = fire;
+  o.n = n;
+  o.p = p + sh;
+  o.s = u.s + k0;
+  o.rho2 = (float)(rr * rr * (1.0 - 0x1p-20));
+  o.err = std::nextafter((float)err, INFINITY);
+  o.lip = (float)(1.01 * lip);
+  o.lip2 = (float)(2.0 * lip2);
+  r = o;
+  return true;
+}
+
+// Adds order c times order b - c of u to order b of its square: the terms kept
+// to (sr, si), the magnitudes of those beyond the degree to w.
+template <int b, int c, int NB>
+inline void add_product(const Poly<NB>& u, const double (*a)[D + 1], double* sr, double* si,
+                        double* w) {
+  constexpr int m = kTerms[c], n = kTerms[b - c], keep = kTerms[b];
+  constexpr bool square = 2 * c == b;
+  const double *yr = u.re[b - c], *yi = u.im[b - c], *ya = a[b - c];
+  for (int i = 0; i < m; i++) {
+    // a square's pairs once: j >= i
+    const int lo = square ? i : 0, mid = std::min(n, std::max(lo, keep - i));
+    const double xr = 2.0 * u.re[c][i], xi = 2.0 * u.im[c][i], xa = 2.0 * a[c][i];
+    for (int j = lo; j < mid; j++) {
+      sr[i + j] += xr * yr[j] - xi * yi[j];
+      si[i + j] += xr * yi[j] + xi * yr[j];
+    }
+    for (int j = mid; j < n; j++) w[i + j] += xa * ya[j];
+    if (square) {  // and the diagonal half
+      if (2 * i < keep) {
+        sr[2 * i] -= 0.5 * (xr * yr[i] - xi * yi[i]);
+        si[2 * i] -= 0.5 * (xr * yi[i] + xi * yr[i]);
+      } else {
+        w[2 * i] -= 0.5 * xa * ya[i];
+      }
+    }
+  }
+  if constexpr (2 * (c + 1) <= b) add_product<b, c + 1>(u, a, sr, si, w);
+}
+
+// One step, u' = 2 X u + F (u^2) + eps (eps_x: of order 0's x, as start jumps
+// have it; else of order 1's constant), over orders [0, nb), and the sums
+// |u_i| |u_j| beyond the degree by order and degree (a: the coefficients'
+// magnitudes).
+template <int b, int NB>
+inline void step_order(const Poly<NB>& u, int nb, const double (*a)[D + 1], double xr, double xi,
+                       double F, Poly<NB>& o, double (*w)[2 * D + 2]) {
+  double sr[D + 1] = {}, si[D + 1] = {};
+  std::fill(w[b], w[b] + 2 * D + 2, 0.0);
+  add_product<b, 0>(u, a, sr, si, w[b]);
+  for (int k = 0; k < kTerms[b]; k++) {
+    o.re[b][k] = 2.0 * (xr * u.re[b][k] - xi * u.im[b][k]) + F * sr[k];
+    o.im[b][k] = 2.0 * (xr * u.im[b][k] + xi * u.re[b][k]) + F * si[k];
+  }
+  if constexpr (b + 1 < NB) {
+    if (b + 1 < nb) step_order<b + 1>(u, nb, a, xr, xi, F, o, w);
+  }
+}
+template <int NB>
+void step_poly(Poly<NB>& u, int nb, const double (*a)[D + 1], double xr, double xi, double F,
+               double eps_x, double (*w)[2 * D + 2]) {
+  Poly<NB> o;
+  o.s = u.s;
+  step_order<0>(u, nb, a, xr, xi, F, o, w);
+  o.re[0][1] += eps_x;
+  if constexpr (NB > 1) {
+    if (nb > 1) o.re[1][0] += 1.0;
+    for (int b = nb; b < NB; b++) {
+      std::fill(o.re[b], o.re[b] + kTerms[b], 0.0);
+      std::fill(o.im[b], o.im[b] + kTerms[b], 0.0);
+    }
+  }
+  u = o;
+}
+
+// With x' = x + theta eps, theta = the constant of order 1 over the linear
+// coefficient, order 1 loses its constant: u(x' - theta eps) re-expanded,
+//   u'_b,k = sum_m (-theta)^m binom(k + m, m) u_{b-m},{k+m},
+// to the terms kept.
+struct Shift {
+  double tr, ti, tm;       // theta, |theta|
+  double d[B + 1][D + 1];  // dropped, by order (the last: beyond the orders) and degree
+  double dp[D + 1];        // |u_0'|
+  double kept[B][D + 1];   // the magnitudes summed in what is kept
+  void recentre(Poly<B>& u, int nb) {
+    const double m2 = u.re[0][1] * u.re[0][1] + u.im[0][1] * u.im[0][1];
+    tr = (u.re[1][0] * u.re[0][1] + u.im[1][0] * u.im[0][1]) / m2;
+    ti = (u.im[1][0] * u.re[0][1] - u.re[1][0] * u.im[0][1]) / m2;
+    tm = norm(tr, ti);
+    Poly<B> o{};
+    o.s = u.s;
+    for (int b = 0; b <= nb; b++) {
+      std::fill(d[b], d[b] + D + 1, 0.0);
+      for (int k = 0; k <= D; k++) {
+        double cr = 1.0, ci = 0.0, cm = 1.0, sr = 0.0, si = 0.0, sm = 0.0;
+        for (int m = 0; m <= b; m++) {
+          if (k + m <= D && b - m < nb && k + m < kTerms[b - m]) {
+            const double x = u.re[b - m][k + m], y = u.im[b - m][k + m];
+            sr += cr * x - ci * y;
+            si += cr * y + ci * x;
+            sm += cm * norm(x, y);
+          }
+          const double f = (double)(k + m + 1) / (m + 1);
+          const double t = -f * (cr * tr - ci * ti);
+          ci = -f * (cr * ti + ci * tr);
+          cr = t;
+          cm *= f * tm;
+        }
+        if (b < nb && k < kTerms[b]) {
+          o.re[b][k] = sr;
+          o.im[b][k] = si;
+        } else {
+          // beyond the orders: a shift of at most 2^-5 of the ball (as the
+          // chain takes), each further one is less than half the one before
+          d[b][k] = b < nb ? sm : 2.0 * sm;
+        }
+        if (b < nb) kept[b][k] = k < kTerms[b] ? sm : 0.0;
+      }
+    }
+    for (int k = 0; k < D; k++) dp[k] = (k + 1) * norm(u.re[0][k + 1], u.im[0][k + 1]);
+    dp[D] = 0.0;
+    o.re[1][0] = o.im[1][0] = 0.0;
+    u = o;
+  }
+  double dropped(int nb, double rho, double eps) const {
+    double s = 0.0;
+    for (int b = nb; b >= 0; b--) s = s * eps + sum_pow(d[b], 0, D, rho);
+    return s;
+  }
+  // The same for any shift, u the polynomial before it: all of the expansion,
+  // sum_b eps^b |u_b|(rho + |theta| eps), less what is kept (and 2^-46 of it for
+  // the difference's own rounding).
+  double dropped_any(const Poly<B>& u, int nb, double rho, double eps) const {
+    double all = 0.0, in = 0.0, a[D + 1];
+    for (int b = nb - 1; b >= 0; b--) {
+      for (int k = 0; k <= D; k++) a[k] = k < kTerms[b] ? norm(u.re[b][k], u.im[b][k]) : 0.0;
+      all = all * eps + sum_pow(a, 0, D, rho + tm * eps);
+      in = in * eps + sum_pow(kept[b], 0, D, rho);
+    }
+    return std::max(0.0, all - in) + 0x1p-46 * all;
+  }
+  // of the terms moved, theta eps u_0' above all
+  double rounding(double rho, double eps) const {
+    return 0x1p-47 * tm * eps * sum_pow(dp, 0, D, rho);
+  }
+};
+
+struct Start {
+  int fire;
+  double hi, lo;  // |eps| of the class's samples, in units of 2^p: (lo, hi]
+};
+
+void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out) {
+  const int f = std::max(1, st.fire - 3) - 1;
+  const int last = od.xlen - 2;
+  if (f < 1 || f >= last) return;
+  Poly<1> u{};
+  {
+    const CFE t[3] = {od.a_fe[f], od.b_fe[f], od.c_fe[f]};
+    u.s = t[0].e + p;  // the linear term's exponent
+    for (int k = 1; k <= 3; k++) {
+      const int e = t[k - 1].e + k * p - u.s;
+      if (e > 900) return;
+      u.re[0][k] = e < -1000 ? 0.0 : std::ldexp(t[k - 1].re, e);
+      u.im[0][k] = e < -1000 ? 0.0 : std::ldexp(t[k - 1].im, e);
+    }
+  }
+  double a[1][D + 1] = {}, w[1][2 * D + 2];
+  for (int k = 1; k <= 3; k++) a[0][k] = norm(u.re[0][k], u.im[0][k]);
+  if (!(a[0][1] > 0.0)) return;
+  double rho[kJumpSubs], R[kJumpSubs], Q[kJumpSubs], P[kJumpSubs];
+  bool alive[kJumpSubs];
+  double x = st.hi;
+  for (int i = 0; i < kJumpSubs; i++) {
+    rho[i] = x;
+    alive[i] = x > 0.0 && (i == 0 || x > st.lo);
+    x *= i < 4 ? 0.84089641525371461 : 0.5;  // 2^-1/4, then octaves
+    R[i] = P[i] = 0.0;
+    // the FP64 path's rounding of its start
+    Q[i] = 0x1p-49 * sum_pow(a[0], 1, 3, rho[i]);
+  }
+  Poly<1> prev = u;
+  double prev_q[kJumpSubs] = {};
+  for (int n = f; n <= last; n++) {
+    if (u.s < -900) return;  // the products below would leave the double range
+    const double xr = od.xhi[n].x, xi = od.xhi[n].y, xm = norm(xr, xi) * (1.0 + 0x1p-50);
+    const double F = pow2(u.s);
+    for (int k = 1; k <= D; k++) a[0][k] = norm(u.re[0][k], u.im[0][k]);
+    bool any = false;
+    for (int i = 0; i < kJumpSubs; i++) {
+      if (!alive[i]) continue;
+      P[i] = sum_pow(a[0], 1, D, rho[i]);
+      const double dmax = (P[i] + R[i] + Q[i]) * F;
+      // the FP64 path has this sample at the same orbit index: it does not
+      // rebase while |delta| < |X| - |delta|, nor bail out below 1000
+      const bool good = R[i] <= kTail * a[0][1] * rho[i] && Q[i] <= 0x1p-20 * a[0][1] * rho[i] &&
+                        xm > 2.1 * dmax && xm + dmax < 1000.0;
+      if (!good || n == last) {
+        alive[i] = false;
+        if (n - 1 - f >= kMinSteps)
+          make_record(prev, st.fire, n - 1, p, rho[i], prev_q[i], 0.0, out[i]);
+        continue;
+      }
+      any = true;
+    }
+    if (!any) return;
+    prev = u;
+    std::copy(Q, Q + kJumpSubs, prev_q);
+    const double eps = pow2(p - u.s);  // eps = x 2^p
+    step_poly(u, 1, a, xr, xi, F, eps, w);
+    for (int i = 0; i < kJumpSubs; i++) {
+      if (!alive[i]) continue;
+      const double h = F * sum_pow(w[0], D + 1, 2 * D, rho[i]);
+      // R: (p + R)^2 = p^2 + (2p + R) R, and p^2's terms beyond the degree
+      R[i] = (2.0 * xm + F * (2.0 * P[i] + R[i])) * R[i] + h;
+      // Q adds, a step: the FP64 path's rounding and its truncated orbit,
+      // 2^-50 (2|X| + |d|)|d| + 2^-52 |eps|; the coefficients' rounding, 2^-50
+      // of 2|X| p for the products and sums, 2^-47 of p^2 for the at most D
+      // products of a convolution, and 2^-51.5 of 2|X| p for the truncated
+      // orbit: 2.36 * 2^-50 of 2|X| p and 9 * 2^-50 of p^2
+      Q[i] = (2.0 * xm + F * (2.0 * P[i] + Q[i])) * Q[i] + h +
+             0x1p-50 * (2.5 * 2.0 * xm * P[i] + 9.5 * F * P[i] * P[i]) + 0x1p-51 * eps * rho[i];
+    }
+    const double big = std::fabs(u.re[0][1]) + std::fabs(u.im[0][1]);
+    if (!(big < 0x1p200) || !(big > 0.0)) return;
+    if (big > 0x1p30 || big < 0x1p-30) {
+      const int sh = std::ilogb(big);
+      for (int k = 1; k <= D; k++) {
+        u.re[0][k] = std::ldexp(u.re[0][k], -sh);
+        u.im[0][k] = std::ldexp(u.im[0][k], -sh);
+      }
+      for (int i = 0; i < kJumpSubs; i++) {
+        R[i] = std::ldexp(R[i], -sh);
+        Q[i] = std::ldexp(Q[i], -sh);
+      }
+      u.s += sh;
+    }
+  }
+}
+
+}  // namespace
+
+void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int threads,
+                       std::vector<JumpRec>& out) {
+  JumpRec none{};
+  none.fire = -1;
+  none.rho2 = -1.0f;
+  out.assign((size_t)kJumpClasses * kJumpSubs, none);
+  if (od.xlen < 64 || !(eps_m > 0.0) || !std::isfinite(eps_m)) return;
+  // |eps| <= hi0 2^p, hi0 in [1/2, 1)
+  const int p = std::ilogb(eps_m) + 1 + eps_e;
+  const double hi0 = std::ldexp(eps_m, -(std::ilogb(eps_m) + 1));
+  // the stop indexes in use, from the outermost samples inward: fire = i for
+  // T_i < |eps|^2 <= T_{i-1}, T the prefix minima of the thresholds
+  auto radius = [&](int i) {  // sqrt(T_i) in units of 2^p (infinite: 4)
+    const RFE& t = od.sa_min_fe[i];
+    if (std::isinf(t.m)) return 4.0;
+    if (!(t.m > 0.0)) return 0.0;
+    const int e = t.e - 2 * p, odd = e & 1;
+    const int k = (e - odd) / 2 + std::ilogb(t.m) / 2;
+    if (k > 4) return 4.0;
+    if (k < -200) return 0.0;
+    return std::sqrt(std::ldexp(t.m, odd)) * pow2((e - odd) / 2);
+  };
+  std::vector<Start> starts;
+  double above = std::min(hi0, radius(1));
+  int i = 1;
+  while ((int)starts.size() < kJumpClasses && above > 0x1p-12) {
+    int lo = i, hi = od.xlen;  // the first index past i with a threshold below `above`
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if (radius(mid) < above)
+        hi = mid;
+      else
+        lo = mid + 1;
+    }
+    if (lo >= od.xlen) break;
+    const double r = radius(lo);
+    starts.push_back({lo, above * (1.0 + 0x1p-16), r});
+    above = r;
+    i = lo;
+  }
+  std::atomic<size_t> next{0};
+  auto work = [&] {
+    for (size_t k; (k = next.fetch_add(1)) < starts.size();)
+      build_class(od, starts[k], p, &out[k * kJumpSubs]);
+  };
+  const size_t nt = std::min(starts.size(), (size_t)std::max(1, threads));
+  std::vector<std::thread> pool;
+  for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
+  work();
+  for (std::thread& t : pool) t.join();
+  // the classes in use first: the device stops at the first unused one, and
+  // knows a class by its first record
+  size_t at = 0;
+  for (size_t k = 0; k < starts.size(); k++) {
+    JumpRec* r = &out[k * kJumpSubs];
+    bool used = false;
+    for (int j = 0; j < kJumpSubs; j++) used |= r[j].fire >= 0;
+    if (!used) continue;
+    for (int j = 0; j < kJumpSubs; j++) r[j].fire = starts[k].fire;
+    if (at != k) std::copy(r, r + kJumpSubs, &out[at * kJumpSubs]);
+    at++;
+  }
+  for (size_t k = at * kJumpSubs; k < out.size(); k++) out[k] = none;
+}
+
+void build_rebase_jumps(const OrbitData& od, double eps_m, int eps_e, std::vector<JumpRec>& out) {
+  constexpr int C = kRebaseClasses;
+  out.clear();
+  const int last = std::min(od.xlen - 2, kRebaseReach);
+  if (last < 2 * kMinSteps || !(eps_m >= 0.0) || !std::isfinite(eps_m)) return;
+  const double eps = eps_e < -1000 ? 0x1p-1000 : std::ldexp(eps_m, eps_e);
+  if (!(eps < 0x1p-16)) return;
+  // an order of eps weighs at most about 2^9 eps over the smallest ball's 2^-43
+  // against the one before: as many as come to 2^-50 (below 2^-110 eps itself
+  // is far under every bound)
+  int nb = 1;
+  if (eps >= 0x1p-110) {
+    const double ratio = std::ldexp(eps, 52);
+    nb = 2;
+    for (double t = ratio * ratio; nb < B && t > 0x1p-50; t *= ratio) nb++;
+  }
+  Poly<B> u{};
+  u.re[0][1] = 1.0;
+  // A sample's FP64 path need not rebase where the FP32 path does: it may hold
+  // the same point as Z' + delta' with |delta'| <= |w| and |Z'| <= 2 |w|, and
+  // then Z' runs along the orbit from Z'^2 + X[0], |Z'|^2 <= 4 |w|^2 <=
+  // 4 (|x| + (1 + |Gamma|) |eps|), which the class kHelper above this one
+  // holds (half of 16 rho0, rho0 the ball before the shifts; classes end below
+  // rho = 4 (1 + |Gamma|) eps).
+  constexpr int kHelper = 4;
+  double rho[C], R[C], Q[C], P[C], E[C], S[C], H[C], T[C], order[B][C], power[2 * B];
+  bool alive[C], open[C];
+  power[0] = 1.0;
+  for (int b = 1; b < 2 * B; b++) power[b] = power[b - 1] * eps;
+  for (int i = 0; i < C; i++) {
+    rho[i] = std::exp2(-0.5 * kRebaseTop - i);
+    R[i] = P[i] = E[i] = 0.0;
+    // the FP64 path's rounding of its first step (delta = 0 * delta + ...)
+    Q[i] = 0x1p-49 * rho[i];
+    alive[i] = true;
+    open[i] = i >= kHelper;
+  }
+  double most = 0.0;
+  double gr = 0.0, gi = 0.0;  // Gamma: x = w^2 + (1 + Gamma) eps
+  JumpRec none{};
+  none.rho2 = -1.0f;
+  out.assign(C, none);
+  Poly<B> prev = u;
+  double prev_q[C] = {}, prev_rho[C] = {}, prev_g[2] = {};
+  double a[B][D + 1] = {}, w[B][2 * D + 2];
+  Shift shift;
+  for (int n = 0; n <= last; n++) {
+    const double xr = od.xhi[n].x, xi = od.xhi[n].y, xm = norm(xr, xi) * (1.0 + 0x1p-50);
+    for (int b = 0; b < nb; b++)
+      for (int k = 0; k < kTerms[b]; k++) a[b][k] = norm(u.re[b][k], u.im[b][k]);
+    const bool end = n == last || !(a[0][D] < 0x1p900) || !(a[0][1] > 0.0);
+    bool any = false;
+    // |delta|'s bounds: the polynomial's sums for the classes down to the first
+    // that is nearly linear (`lin`).  From there on a smaller ball's nonlinear
+    // part is at most the square of the ratio of the radii times that one's, an
+    // order of eps its constant and the rest times the ratio.
+    int first = 0;
+    while (first < C - 1 && !alive[first]) first++;
+    int lin = C - 1;
+    for (int i = first; i < C; i++) {  // (a guess by the first two terms)
+      if (a[0][2] * rho[i] < 0x1p-14 * a[0][1]) {
+        lin = i;
+        break;
+      }
+    }
+    const int full = lin - first + 1;
+    sums_pow(a[0], 1, D, rho + first, full, P + first);
+    for (int i = first; i <= lin; i++) E[i] = 0.0;
+    double flat = 0.0;
+    for (int b = nb - 1; b > 0; b--) {
+      sums_pow(a[b], 0, kTerms[b] - 1, rho + first, full, S + first);
+      for (int i = first; i <= lin; i++) {
+        E[i] = (E[i] + S[i]) * eps;
+        order[b][i] = S[i];
+      }
+      flat = (flat + a[b][0]) * eps;
+    }
+    const double bend = P[lin] - a[0][1] * rho[lin] + 0x1p-50 * P[lin];
+    const double slope = E[lin] * (1.0 + 0x1p-50) - flat;
+    for (int i = lin + 1; i < C; i++) {
+      const double t = rho[i] / rho[lin];
+      P[i] = a[0][1] * rho[i] + bend * t * t;
+      E[i] = flat + slope * t;
+    }
+    // a ball's own bound on |delta| holds while R is a small part of it
+    for (int i = 0; i < C; i++)
+      if (alive[i] && !(R[i] <= 0x1p-6 * P[i])) alive[i] = false;
+    for (int i = 0; i < C; i++) {
+      if (!open[i]) continue;
+      const int h = i - kHelper;
+      const double d = P[i] + E[i] + R[i] + Q[i];
+      // |delta'| in the FP64 path's representation, |Z'| <= |X| + its helper's
+      const double d2 = alive[h] ? d + P[h] + E[h] + R[h] : INFINITY;
+      const bool good = alive[i] && !end && R[i] <= kTail * a[0][1] * rho[i] &&
+                        Q[i] <= 0x1p-20 * a[0][1] * rho[i] && xm > d + 1.1 * d2 &&
+                        xm + d2 < 1000.0;
+      if (good) {
+        any = true;
+        continue;
+      }
+      open[i] = false;
+      if (n - 1 < kMinSteps) continue;
+      // the record's own Gamma, which takes the constant of order 1 out
+      Poly<B> at = prev;
+      double r = prev_rho[i], q = prev_q[i];
+      shift.tr = shift.ti = 0.0;
+      if (nb > 1) {
+        shift.recentre(at, nb);
+        if (shift.tm * eps < 0x1p-3 * r) {
+          r -= shift.tm * eps;
+          q += shift.dropped_any(prev, nb, r, eps) + shift.rounding(r, eps);
+        } else {
+          at = prev;
+          shift.tr = shift.ti = 0.0;
+        }
+      }
+      if (!make_record(at, 0, n - 1, 0, r, q, nb > 1 ? eps : 0.0, out[i])) continue;
+      const double g1 = 1.0 + prev_g[0] + shift.tr, g2 = prev_g[1] + shift.ti;
+      Flt4& g = out[i].gamma;
+      g.x = (float)g1;
+      g.y = (float)(g1 - (double)g.x);
+      g.z = (float)g2;
+      g.w = (float)(g2 - (double)g.z);
+    }
+    if (!any) break;
+    prev = u;
+    std::copy(Q, Q + C, prev_q);
+    std::copy(rho, rho + C, prev_rho);
+    prev_g[0] = gr;
+    prev_g[1] = gi;
+    step_poly(u, nb, a, xr, xi, 1.0, 0.0, w);
+    // the square's terms beyond the degrees (order b's scale with a ball's radius
+    // to the kTerms[b] at least) and beyond the orders
+    sums_pow(w[0], D + 1, 2 * D, rho + first, full, H + first);
+    for (int i = first; i <= lin; i++) T[i] = 0.0;
+    for (int b = nb - 1; b >= 1; b--) {
+      sums_pow(w[b], kTerms[b], 2 * D, rho + first, full, S + first);
+      for (int i = first; i <= lin; i++) T[i] = (T[i] + S[i]) * eps;
+    }
+    for (int i = first; i <= lin; i++) {
+      double x = nb == 1 ? eps : 0.0;
+      for (int b = 1; b < nb; b++)
+        for (int c = nb - b; c < nb; c++) x += order[b][i] * order[c][i] * power[b + c];
+      H[i] += T[i];
+      T[i] = x;
+    }
+    for (int i = 0; i < C; i++) {
+      if (!alive[i]) continue;
+      const double t = i > lin ? rho[i] / rho[lin] : 1.0;
+      const double h = i > lin ? H[lin] * t * t + T[lin] : H[i] + T[i];
+      const double d = P[i] + E[i];
+      R[i] = (2.0 * xm + 2.0 * d + R[i]) * R[i] + h;
+      const int hh = i - kHelper;
+      // the FP64 path's step at |Z'| <= |X| + d_h, |delta'| <= d + d_h
+      const double dh = hh >= 0 && alive[hh] ? P[hh] + E[hh] + R[hh] : 0.0;
+      Q[i] = (2.0 * xm + 2.0 * d + Q[i]) * Q[i] + h +
+             0x1p-50 * (2.0 * xm + 3.0 * (d + dh)) * (d + dh) +
+             0x1p-50 * (1.5 * 2.0 * xm * d + 8.5 * d * d) + 0x1p-48 * eps;
+    }
+    if (nb == 1) continue;
+    // Recentre (Shift) where the linear coefficient is the largest so far:
+    // theta goes with its inverse, and after a near return of the orbit it is
+    // small for a while.
+    const double m = u.re[0][1] * u.re[0][1] + u.im[0][1] * u.im[0][1];
+    if (!(m > most) || !(m < 1e300)) continue;
+    // (a constant far below every ball stays)
+    if (norm(u.re[1][0], u.im[1][0]) * eps < 0x1p-16 * rho[C - 1] * std::sqrt(m)) continue;
+    most = m;
+    shift.recentre(u, nb);
+    gr += shift.tr;
+    gi += shift.ti;
+    for (int i = 0; i < C; i++) {
+      if (!alive[i]) continue;
+      const double r = shift.dropped(nb, rho[i], eps);
+      R[i] += r;
+      Q[i] += r + shift.rounding(rho[i], eps);
+      rho[i] -= shift.tm * eps;
+      // (see Shift::dropped), and half of it in all
+      if (rho[i] < 0.5 * std::exp2(-0.5 * kRebaseTop - i) ||
+          rho[i] < 4.0 * (1.0 + norm(gr, gi)) * eps || shift.tm * eps > 0x1p-5 * rho[i])
+        alive[i] = false;
+    }
+  }
+}
+
+}  // namespace nmg

@@ -63,6 +63,33 @@ struct TFE {               // m * 2^e, m in [1, 2); e = kTfeInf: +inf, kTfeZero:
 };
 constexpr int32_t kTfeInf = 0x7fffffff, kTfeZero = -0x7fffffff;
 
+// A jump of the FP32 path (jump.hpp): for start values |x|^2 <= rho2 in units
+// of 2^2p,
+//     delta_n = 2^s (b[0] x + ... + c[..] x^kJumpDegree
+//                    + e (q1[0] + q1[1] x + ...) + e^2 (q2[0] + ...) + ...),
+// e = 2^32 eps, within err 2^s, the distance of the FP64 path's own delta_n
+// included.
+constexpr int kJumpDegree = 16;
+constexpr int kJumpExact = 7;     // terms in float-float; the rest in FP32
+constexpr int kJumpOrders = 5;    // orders of eps (rebase jumps), with terms
+constexpr int kJumpEps1 = 8, kJumpEps2 = 5, kJumpEps3 = 3, kJumpEps4 = 2;
+constexpr int kJumpClasses = 12;  // series stop indexes
+constexpr int kJumpSubs = 7;      // radii of each
+constexpr int kRebaseClasses = 36;
+constexpr int kRebaseTop = 16;    // class i: |x|^2 < 2^-(kRebaseTop + 2 i)
+struct Flt2 {
+  float x, y;
+};
+struct alignas(16) JumpRec {
+  int32_t fire, n, p, s;
+  float rho2, err, lip, lip2;  // bounds of |d delta_n / dx| and of half its second
+  Flt4 gamma;          // 1 + Gamma (rebase jumps)
+  Flt4 b[kJumpExact];  // {re.h, re.l, im.h, im.l}, as gamma
+  Flt2 c[kJumpDegree - kJumpExact];
+  // of (2^32 eps)^1 .. (2^32 eps)^4
+  Flt2 q1[kJumpEps1], q2[kJumpEps2], q3[kJumpEps3], q4[kJumpEps4];
+};
+
 enum CardioidMode : int32_t {
   CARDIOID_PER_SAMPLE = 0,  // evaluate the test for each sample (double-double)
   CARDIOID_NONE = 1,        // the view box is provably outside both regions
@@ -117,6 +144,8 @@ struct DeviceView {
   const CFFE* sa_b32;
   const CFFE* sa_c32;
   const TFE* sa_min32;     // [xlen]
+  const JumpRec* jump;     // [kJumpClasses * kJumpSubs], then [kRebaseClasses]; or null
+  float jump_w2;           // rebases with |w|^2 below it may jump (0: none)
 
   // the reference-exact path: values in the view's arbitrary precision as
   // records of mp_limbs limbs (mpf_fixed.cuh; word 0: exponent << 32 | sign)
