@@ -299,17 +299,18 @@ void build_jump_tables(nm_handle* h, int threads) {
     for (const nmg::RFE& y : h->eps_im_fe) my = std::max(my, std::fabs(std::scalbn(y.m, y.e - e)));
   }
   const double m = std::sqrt(mx * mx + my * my) * (1.0 + 0x1p-40);
-  nmg::build_start_jumps(h->od, m, e, threads, h->jump);
-  std::vector<nmg::JumpRec> re;
-  nmg::build_rebase_jumps(h->od, m, e, re);
-  nmg::JumpRec none{};
-  none.rho2 = -1.0f;
-  re.resize(nmg::kRebaseClasses, none);
-  // a rebase may jump when x = w^2 + (1 + Gamma) eps lies in a class in use
-  h->jump_w2 = 0.0f;
-  for (int i = 0; i < nmg::kRebaseClasses && h->jump_w2 == 0.0f; i++)
-    if (re[i].rho2 > 0.0f) h->jump_w2 = (float)std::exp2(-0.5 * nmg::kRebaseTop - i);
-  h->jump.insert(h->jump.end(), re.begin(), re.end());
+  nmg::JumpTables t;
+  nmg::build_jumps(h->od, m, e, threads, t);
+  h->jump = std::move(t.start);
+  h->jump.insert(h->jump.end(), t.chain.begin(), t.chain.end());
+  h->jump_x2 = 0.0f;
+  for (int k = 0; k < nmg::kChains; k++) {
+    // X[s] is z[s + 1]
+    h->jump_from[k] = t.start_index[k] < 0 ? -1 : t.start_index[k] + 1;
+    for (int i = 0; i < nmg::kChainClasses; i++)
+      if (t.chain[(size_t)k * nmg::kChainClasses + i].rho2 > 0.0f)
+        h->jump_x2 = std::max(h->jump_x2, (float)std::exp2(-nmg::kChainTop - 2 * i));
+  }
 }
 
 int check_handle(const nm_handle* h) {
@@ -329,7 +330,8 @@ void set_fe_tables(const nm_handle* h, nmg::DeviceView& v) {
     v.sa_c32 = t->d_c32.p;
     v.sa_min32 = t->d_sa_min32.p;
     v.jump = t->jump.empty() ? nullptr : t->d_jump.p;
-    v.jump_w2 = t->jump_w2;
+    std::copy(t->jump_from, t->jump_from + nmg::kChains, v.jump_from);
+    v.jump_x2 = t->jump_x2;
   }
   v.sa_fe = h->od.sa_fp64_ok ? 0 : 1;
   if (!v.sa_fe) return;
@@ -479,7 +481,8 @@ nm_handle* nm_copy(const nm_handle* src) {
   h->c32 = src->c32;
   h->sa_min32 = src->sa_min32;
   h->jump = src->jump;
-  h->jump_w2 = src->jump_w2;
+  std::copy(src->jump_from, src->jump_from + nmg::kChains, h->jump_from);
+  h->jump_x2 = src->jump_x2;
   h->reference_mode = src->reference_mode;
   h->fe_single_pass = src->fe_single_pass;
   h->fe_overlap = src->fe_overlap;

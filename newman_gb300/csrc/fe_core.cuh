@@ -83,6 +83,21 @@ __device__ __forceinline__ FF fe_twice_plus(float ah, float al, FF b) {
 // 2 (2^-20 (|Z| + |delta|) + e + u_z |Z| + u (|Z| + |delta|)), stays below
 // 2 (0.0043 + e + 2^-30) < 0.49 <= 1024 - |Y| whenever e < 0.2.
 constexpr float kFeQuickErr = 0.2f;
+// The same for a state with |Y|^2 <= 2^18, half the bailout radius: the band stays
+// below 2 (0.0043 + e + 2^-30) < 512 <= 1024 - |Y| whenever e < 200.  A sample's
+// bound often passes 0.2 some twenty steps before its escape, and with 32 lanes
+// a warp then took the full test on nearly every step.
+constexpr float kFeQuickErrInner = 200.0f;
+constexpr float kFeInner2 = 262144.0f;
+
+// A rebase test |Y|^2 < |delta|^2 nearer to a tie than this may come out unlike in
+// FP32 and FP64: the sample ends uncertified, so that on the others both paths
+// rebase at the same steps for as long as their bound is small.  (The estimates
+// are within 2^-20; a bound of 2^-23 |delta| on each path moves the squares by
+// 2^-20.)  With a
+// larger bound a sample no longer jumps (fe_chain_jump).
+constexpr float kFeTie = 0x1p-19f;
+constexpr float kFeTied = 0x1p-46f;  // ... while the bound is below 2^-23 |delta|
 
 // Interior orbits on double-loop views.  The reference's double loop F (one
 // step z -> z^2 + c in doubles, mandelbrot.cpp:242-246) rounds by at most
@@ -255,9 +270,8 @@ __device__ __forceinline__ TFE tfe_norm(float m, int e) {
 }
 
 // The polynomial of a jump's record at x (in its units), without the eps part,
-// times 2^-s: the first kJumpExact terms in float-float, the rest in FP32 (a
-// term's size falls by 2^-3 or more a degree, so their rounding is below the
-// float-float terms').
+// times 2^-s: the first kJumpExact terms in float-float, the rest in FP32 (their
+// rounding is in the record's bound).
 __device__ __forceinline__ void jump_poly(const JumpRec& rec, FF xr, FF xi, FF& dr, FF& di) {
   constexpr int n = kJumpDegree - kJumpExact;
   float hr = rec.c[n - 1].x, hi = rec.c[n - 1].y;
@@ -446,7 +460,12 @@ __device__ __forceinline__ FF ff_norm2(FF x, FF y) {
 
 // The bailout test on Y = Z + delta (unscaled, float-float).  Returns true
 // when |Y|^2 > 2^20; clears `certified` when the error bound `yerr` on |Y|
-// reaches across 1024.
+// reaches across 1024, or (kSmooth) when an escaped sample's exceeds |Y| / 4: the
+// smoothing term moves by up to 0.21 of the relative error of |Y|, and a bound of
+// |Y| itself let it differ from the FP64 path's by 4e-4 (the 3840x2160 view at
+// 1e-300, one sample in 3 million) where this lets it by 2e-4, for 7 % more
+// reworked samples.
+template <bool kSmooth>
 __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& certified,
                                                FF& r2) {
   r2 = ff_norm2(yr, yi);
@@ -454,6 +473,7 @@ __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& c
   // | |Y| - 1024 | <= 2 yerr  <=>  | |Y|^2 - 2^20 | <= (2048 + 2 yerr) 2 yerr
   if (fabsf(d) <= up_fma(up_fma(2.0f, yerr, 2048.0f), up_mul(2.0f, yerr), up_mul(0x1p-40f, r2.h)))
     certified = false;
+  if (kSmooth && d > 0.0f && up_mul(16.0f * yerr, yerr) > r2.h) certified = false;
   return d > 0.0f;
 }
 
@@ -485,47 +505,58 @@ __device__ __forceinline__ void fe_renormalise(FeState& st) {
   }
 }
 
-// The jump (jump.hpp) of a sample that has just rebased (j = 0, delta = Y = w):
-// its next n + 1 steps at once, where w^2 + (1 + Gamma) eps lies in the ball of
-// a record.  The bound passes through the jump by the polynomial's derivative
-// bound: e' = 2|w| e + e^2 + rounding of x, e'' = lip e' + err.
-__device__ __forceinline__ void fe_rebase_jump(const DeviceView& v, FeState& st) {
-  const float wl1 = up_add(fabsf(st.dr.h), fabsf(st.di.h));
-  if (!(fmaf(st.dr.h, st.dr.h, st.di.h * st.di.h) < v.jump_w2)) return;
-  // class i: |x|^2 < 2^-(kRebaseTop + 2 i), i from the exponent of |w^2 + eps|^2
-  const float ar = fmaf(st.dr.h, st.dr.h, fmaf(-st.di.h, st.di.h, st.er.h));
-  const float ai = fmaf(2.0f * st.dr.h, st.di.h, st.ei.h);
-  int i = (126 - kRebaseTop - (__float_as_int(fmaf(ar, ar, ai * ai)) >> 23)) >> 1;
-  const JumpRec* base = v.jump + kJumpClasses * kJumpSubs;
+// The chain a sample at orbit index j with delta small may jump along, or -1.
+__device__ __forceinline__ int fe_chain_at(const DeviceView& v, int j) {
+  int k = -1;
+#pragma unroll
+  for (int c = 0; c < kChains; c++)
+    if (j == v.jump_from[c]) k = c;
+  return k;
+}
+
+// The jump (jump.hpp) of a sample at a chain's first index: its next steps at
+// once, where x = delta + Gamma eps lies in the ball of a record.  The bound
+// passes through the jump by the polynomial's derivative at x: e' = |d delta/dx| e
+// + err.  A bound above 2^-24 |x| keeps the sample from jumping: below it
+// every rebase so far was decided alike in both paths (kFeTie).
+__device__ __forceinline__ void fe_chain_jump(const DeviceView& v, FeState& st) {
+  const int c = fe_chain_at(v, st.j);
+  if (c < 0) return;
+  const float x2 = fmaf(st.dr.h, st.dr.h, st.di.h * st.di.h);
+  if (!(x2 < v.jump_x2)) return;
+  // class i: |x|^2 < 2^-(kChainTop + 2 i), i from the exponent of |delta|^2
+  int i = (126 - kChainTop - (__float_as_int(x2) >> 23)) >> 1;
+  const JumpRec* base = v.jump + kJumpClasses * kJumpSubs + c * kChainClasses;
   const FF zero{0.0f, 0.0f};
   const JumpRec* use = nullptr;
   FF sr = zero, si = zero;
+  const bool with_eps = fabsf(st.er.h) + fabsf(st.ei.h) > 0x1p-110f;
   // its own class, or up to two larger ones (below the smallest class its bound
   // would be far above delta's own scale)
   for (int t = 0; t < 3 && !use; t++, i--) {
     if (i < 0) return;
-    if (i >= kRebaseClasses || !(base[i].rho2 > 0.0f)) continue;
-    // x = w^2 + (1 + Gamma) eps, in the record's units
-    const Flt4 g = base[i].gamma;
-    FF gr, gi, xr, xi;
-    ff_cmul_add(st.er, st.ei, FF{g.x, g.y}, FF{g.z, g.w}, zero, zero, gr, gi);
-    ff_cmul_add(st.dr, st.di, st.dr, st.di, gr, gi, xr, xi);
-    sr = ff_scale(xr, -base[i].p);
-    si = ff_scale(xi, -base[i].p);
+    if (i >= kChainClasses || !(base[i].rho2 > 0.0f)) continue;
+    // x = delta + Gamma eps, in the record's units
+    FF xr = st.dr, xi = st.di;
+    if (with_eps) {
+      const Flt4 g = base[i].gamma;
+      ff_cmul_add(st.er, st.ei, FF{g.x, g.y}, FF{g.z, g.w}, st.dr, st.di, xr, xi);
+    }
+    const float u = base[i].unit;
+    sr = FF{xr.h * u, xr.l * u};
+    si = FF{xi.h * u, xi.l * u};
     if (fmaf(sr.h, sr.h, si.h * si.h) <= base[i].rho2) use = base + i;
   }
   if (!use) return;
-  const int n = use->n, p = use->p, s = use->s;
-  if (st.i + n + 1 >= v.N) return;
-  // bound of x: 2 |w| e + e^2 and the products' rounding (|w| as in a step, to
-  // 2^-20 of it: a looser norm would compound over a sample's jumps)
+  const int n = use->n - use->fire;  // steps
+  if (st.i + n >= v.N) return;
+  // bound of x: delta's, and the product's rounding
   const float el1 = up_add(fabsf(st.er.h), fabsf(st.ei.h));
   const float gl1 = up_add(fabsf(use->gamma.x), fabsf(use->gamma.z));
-  const float wn = up_fma(0x1p-20f, wl1, approx_norm(st.dr.h, st.di.h));
-  float ex = up_fma(up_fma(2.0f, wn, st.err), st.err, up_mul(kFeU, up_mul(wl1, wl1)));
-  ex = up_fma(up_mul(4.0f * kFeU, gl1), el1, ex);
-  ex = up_add(ldexpf(ex, -p), 0x1p-100f);
-  if (!(ex < 0x1p-12f)) return;
+  const float xl1 = up_add(fabsf(st.dr.h), fabsf(st.di.h));
+  float ex = up_fma(kFeU, up_fma(up_mul(2.0f, gl1), el1, xl1), st.err);
+  ex = up_add(up_mul(ex, use->unit), 0x1p-100f);
+  if (!(ex * ex < 0x1p-48f * fmaf(sr.h, sr.h, si.h * si.h))) return;
   FF dr, di;
   jump_poly(*use, sr, si, dr, di);
   // the orders of eps, and |d delta / dx| at x, in FP32
@@ -540,7 +571,7 @@ __device__ __forceinline__ void fe_rebase_jump(const DeviceView& v, FeState& st)
     }
   };
   const float er = st.er.h * 0x1p32f, ei = st.ei.h * 0x1p32f;
-  if (fabsf(er) + fabsf(ei) > 0x1p-78f) {
+  if (with_eps) {
     float qr, qi, tr, ti;
     auto times_eps = [&]() {
       const float t = fmaf(qr, er, -qi * ei);
@@ -557,31 +588,49 @@ __device__ __forceinline__ void fe_rebase_jump(const DeviceView& v, FeState& st)
     qr += tr;
     qi += ti;
     times_eps();
-    horner(use->q1, kJumpEps1, tr, ti);
-    qr += tr;
-    qi += ti;
-    times_eps();
-    dr = ff_add(dr, FF{qr, 0.0f});
-    di = ff_add(di, FF{qi, 0.0f});
+    // order 1: its first terms in float-float (2^-17 of delta on the 1e-12 view),
+    // the later ones and the orders above in FP32
+    horner(use->q1 + kEpsExact, kJumpEps1 - kEpsExact, tr, ti);
+    const float ur = fmaf(tr, xh, -ti * yh), ui = fmaf(tr, yh, ti * xh);
+    FF or_{ur, 0.0f}, oi{ui, 0.0f};
+#pragma unroll 1
+    for (int k = kEpsExact - 1; k >= 0; k--) {
+      const Flt2 c = use->q1[k], l = use->q1l[k];
+      or_ = ff_add(or_, FF{c.x, l.x});
+      oi = ff_add(oi, FF{c.y, l.y});
+      if (k > 0) {
+        FF nr, ni;
+        ff_cmul_add(or_, oi, sr, si, zero, zero, nr, ni);
+        or_ = nr;
+        oi = ni;
+      }
+    }
+    or_ = ff_add(or_, FF{qr, 0.0f});
+    oi = ff_add(oi, FF{qi, 0.0f});
+    const FF er2{er, st.er.l * 0x1p32f}, ei2{ei, st.ei.l * 0x1p32f};
+    FF nr, ni;
+    ff_cmul_add(or_, oi, er2, ei2, dr, di, nr, ni);
+    dr = nr;
+    di = ni;
   }
   float gr = 0.0f, gi = 0.0f;
 #pragma unroll
-  for (int k = kJumpDegree; k >= 1; k--) {
-    const float cr = k > kJumpExact ? use->c[k - kJumpExact - 1].x : use->b[k - 1].x;
-    const float ci = k > kJumpExact ? use->c[k - kJumpExact - 1].y : use->b[k - 1].z;
-    const float t = fmaf(gr, xh, fmaf(-gi, yh, (float)k * cr));
-    gi = fmaf(gr, yh, fmaf(gi, xh, (float)k * ci));
+  for (int k = kJumpDegree - 1; k >= 0; k--) {
+    const Flt2 c = use->d[k];
+    const float t = fmaf(gr, xh, fmaf(-gi, yh, c.x));
+    gi = fmaf(gr, yh, fmaf(gi, xh, c.y));
     gr = t;
   }
   // FP32 rounding of it (at most 2^-18 of the sum of its terms) and the second
   // derivative over the ball of radius ex
   const float amp = up_fma(use->lip2, ex, up_fma(0x1p-17f, use->lip, approx_norm(gr, gi)));
   const float err = up_fma(amp, ex, use->err);
-  st.dr = ff_scale(dr, s);
-  st.di = ff_scale(di, s);
-  st.err = up_add(ldexpf(err, s), 0x1p-120f);
-  st.j = n + 1;
-  st.i += n + 1;
+  const float sc = use->scale;
+  st.dr = FF{dr.h * sc, dr.l * sc};
+  st.di = FF{di.h * sc, di.l * sc};
+  st.err = up_add(up_mul(err, sc), 0x1p-120f);
+  st.j += n;
+  st.i += n;
 }
 
 // Steps while delta is scaled: Y = Z to working precision, so the events are
@@ -639,7 +688,7 @@ __device__ __forceinline__ bool fe_scaled_steps(const DeviceView& v, FeState& st
                                 up_mul(kFeUZ, up_add(fabsf(z.hx), fabsf(z.hy))));
       bool cert = st.certified != 0;
       FF r2;
-      if (fe_escape_test(yr, yi, yerr, cert, r2)) {
+      if (fe_escape_test<true>(yr, yi, yerr, cert, r2)) {
         st.certified = cert ? 1 : 0;
         res.it = st.i;
         res.r2 = r2;
@@ -744,7 +793,8 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
     // view (whose second bound e64 is propagated every step), at the orbit's
     // last point, or once the bound has grown past kFeQuickErr; otherwise it
     // is decided (|Y| below 1024 by more than the band) -- see kFeQuickErr.
-    if (dloop || r2 > lo_band || !(err < kFeQuickErr) || j == zlast) {
+    if (dloop || r2 > lo_band ||
+        !(err < (r2 <= kFeInner2 ? kFeQuickErrInner : kFeQuickErr)) || j == zlast) {
       const float zn1 = up_add(fabsf(z.hx), fabsf(z.hy)), dn1 = up_add(fabsf(dr.h), fabsf(di.h));
       float yerr = y_err();
       if (dloop) {
@@ -779,8 +829,8 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
         }
       } else {
         FF r2ff;
-        if (fe_escape_test(ff_add(FF{z.hx, z.lx}, dr), ff_add(FF{z.hy, z.ly}, di), yerr,
-                           certified, r2ff)) {
+        if (fe_escape_test<!kDl>(ff_add(FF{z.hx, z.lx}, dr), ff_add(FF{z.hy, z.ly}, di), yerr,
+                                 certified, r2ff)) {
           res.it = i;
           res.r2 = r2ff;
           done = true;
@@ -795,26 +845,31 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
       }
     }
     const float d2 = fmaf(dr.h, dr.h, di.h * di.h);
-    // A rebase is open at any step (delta = Y against Z[0] is the same point,
-    // its rounding in the bound); taken early, up to |Y| = 4 |delta|, where Y
-    // is small enough to jump from: the orbit's own near returns to 0 then end
-    // in a rebase for every sample.
-    const bool small = !kDl && r2 < v.jump_w2;
-    if (r2 < (small ? 16.0f * d2 : d2) || j == zlast) {  // rebase to Z[0]: delta = Y in float-float
-      const float yerr_fe = y_err();
-      const FF nyr = ff_add(FF{z.hx, z.lx}, dr);
-      const FF nyi = ff_add(FF{z.hy, z.ly}, di);
-      dr = nyr;
-      di = nyi;
-      err = yerr_fe;
-      j = 0;
-      z = fe_load_z<kStaged>(v, 0);
-      ym = approx_norm(dr.h, di.h);
-      rebases++;
-      if (small) {  // jumps with the other lanes' at the next chunk's start
+    if (r2 < (kDl ? d2 : d2 * (1.0f + kFeTie)) || j == zlast) {
+      if (!kDl && j != zlast && r2 >= d2 * (1.0f - kFeTie) && err * err < kFeTied * d2) {
+        certified = false;
+        done = true;
         i++;
         break;
       }
+      if (r2 < d2 || j == zlast) {  // rebase to Z[0]: delta = Y in float-float
+        const float yerr_fe = y_err();
+        const FF nyr = ff_add(FF{z.hx, z.lx}, dr);
+        const FF nyi = ff_add(FF{z.hy, z.ly}, di);
+        dr = nyr;
+        di = nyi;
+        err = yerr_fe;
+        j = 0;
+        z = fe_load_z<kStaged>(v, 0);
+        ym = approx_norm(dr.h, di.h);
+        rebases++;
+      }
+    }
+    // at a chain's first index with delta small: jumps with the other lanes' at
+    // the next round's start
+    if (!kDl && d2 < v.jump_x2 && fe_chain_at(v, j) >= 0) {
+      i++;
+      break;
     }
   }
   if (kDl && trap && !done && certified && i < v.N) {
@@ -881,10 +936,41 @@ __device__ __forceinline__ bool fe_advance(const DeviceView& v, FeState& st, int
     }
     return fe_scaled_steps<kStaged, kRawT>(v, st, steps, res, executed, rebases);
   }
-  if (!v.double_loop && st.j == 0) fe_rebase_jump(v, st);
   if (v.double_loop)
     return fe_unscaled_steps<true, kStaged, kRawT>(v, st, steps, res, executed, rebases, trap);
   return fe_unscaled_steps<false, kStaged, kRawT>(v, st, steps, res, executed, rebases, nullptr);
+}
+
+// A sample at a chain's first index with delta small: it may jump.
+__device__ __forceinline__ bool fe_may_jump(const DeviceView& v, const FeState& st) {
+  return !v.double_loop && st.E == 0 &&
+         fmaf(st.dr.h, st.dr.h, st.di.h * st.di.h) < v.jump_x2 && fe_chain_at(v, st.j) >= 0;
+}
+
+// One round of a warp's samples, for the persistent loops: the jumps of every
+// lane that may, together, then bursts of kFeBurst steps (advance(n))
+// until `chunk` steps are done or kFeIdle lanes stand idle -- finished, about
+// to jump, or empty.  A jump costs a warp about seven steps' instructions
+// whether one lane or all take it, and a refill or a finished sample's store
+// one: they wait for company, but a waiting lane is idle.  Double-loop views
+// step the chunk in one go (their trapping test runs once a call).  Every lane
+// of the warp calls it; true, per lane, when its sample is finished.
+constexpr int kFeBurst = 16;
+constexpr int kFeIdle = 10;
+template <class Advance>
+__device__ __forceinline__ bool fe_round(const DeviceView& v, FeState& st, bool active, int chunk,
+                                         Advance advance) {
+  const unsigned kFull = 0xffffffffu;
+  bool run = active, done = false;
+  if (active && fe_may_jump(v, st)) fe_chain_jump(v, st);
+  for (int left = chunk; left > 0; left -= kFeBurst) {
+    if (run) {
+      done = advance(v.double_loop ? chunk : min(left, kFeBurst));
+      run = !done && !v.double_loop && !fe_may_jump(v, st);
+    }
+    if (__popc(__ballot_sync(kFull, run)) <= 32 - kFeIdle) break;
+  }
+  return done;
 }
 
 }  // namespace nmg

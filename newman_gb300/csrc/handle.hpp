@@ -114,7 +114,8 @@ struct nm_handle {
   std::vector<nmg::CFFE> a32, b32, c32;
   std::vector<nmg::TFE> sa_min32;
   std::vector<nmg::JumpRec> jump;
-  float jump_w2 = 0.0f;
+  int32_t jump_from[nmg::kChains] = {};
+  float jump_x2 = 0.0f;
   DevBuf<nmg::FFE> d_eps32_re, d_eps32_im;
   DevBuf<nmg::CFFE> d_a32, d_b32, d_c32;
   DevBuf<nmg::TFE> d_sa_min32;

@@ -14,7 +14,7 @@ namespace nmg {
 namespace {
 
 constexpr int D = kJumpDegree;
-// Orders of eps (rebase jumps) and the terms x^0 .. of each: order 0 has x^1 ..
+// Orders of eps (chain jumps) and the terms x^0 .. of each: order 0 has x^1 ..
 // x^D, the others what FP32 holds of them (JumpRec).
 constexpr int B = kJumpOrders;
 constexpr int kTerms[B] = {D + 1, kJumpEps1, kJumpEps2, kJumpEps3, kJumpEps4};
@@ -22,12 +22,12 @@ constexpr int kTerms[B] = {D + 1, kJumpEps1, kJumpEps2, kJumpEps3, kJumpEps4};
 // step, and since R grows by 2^D an octave of delta, a tighter or looser limit
 // moves the target by a few steps only.
 constexpr double kTail = 0x1p-46;
-// A record is worth its evaluation (seven float-float multiply-adds and two
-// dozen plain ones, four steps' work, and a lane's wait for its warp) from here on.
+// A record is worth its evaluation (four steps' work and a lane's wait for
+// its warp) from here on.
 constexpr int kMinSteps = 16;
 
-// A rebase jump goes at most this far.
-constexpr int kRebaseReach = 4096;
+// A chain's jumps go at most this far.
+constexpr int kChainReach = 4096;
 
 double norm(double re, double im) { return std::sqrt(re * re + im * im); }
 
@@ -76,6 +76,7 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
     const double im = std::ldexp(u.im[0][k], sh * k - k0);
     const double m = norm(re, im);
     lip += k * m * rk;
+    o.d[k - 1] = {(float)(k * re), (float)(k * im)};
     if (k > 1) lip2 += 0.5 * k * (k - 1) * m * rk / rr;
     rk *= rr;
     if (!(m < 0x1p100)) return false;
@@ -91,11 +92,11 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
       b.z = (float)im;
       b.w = (float)(im - (double)b.z);
     } else {
-      // plain FP32: coefficient, operand and each of the at most 2 D roundings
-      // of the Horner chain within 2^-24 of at most twice the terms' sum
       o.c[k - kJumpExact - 1] = {(float)re, (float)im};
-      err += 0x1p-18 * m * rk;
     }
+    // plain FP32: the coefficient, x^k, and at most 3 of 2^-24 a Horner step on
+    // the partial sums it is part of
+    if (k > kJumpExact) err += (8.0 + 4.0 * k) * 0x1p-24 * m * rk;
   }
   // the orders of eps in plain FP32, coefficients times 2^-32b for (2^32 eps)^b
   Flt2* const tab[B] = {nullptr, o.q1, o.q2, o.q3, o.q4};
@@ -107,7 +108,11 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
       const double m = norm(re, im);
       if (!(m < 0x1p100)) return false;
       tab[b][k] = {(float)re, (float)im};
-      err += (0x1p-18 * m + 0x1p-100) * rk;
+      const bool ff = b == 1 && k < kEpsExact;
+      if (ff) o.q1l[k] = {(float)(re - (double)(float)re), (float)(im - (double)(float)im)};
+      // rounded: the coefficient, y^k, at most 3 of 2^-24 a Horner step on the
+      // partial sums it is part of, and the product and sum with the next order
+      err += ((8.0 + 4.0 * (k + 2.0 * b)) * (ff ? 0x1p-43 : 0x1p-24) * m + 0x1p-100) * rk;
       rk *= rr;
     }
   }
@@ -131,6 +136,8 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
   o.n = n;
   o.p = p + sh;
   o.s = u.s + k0;
+  o.unit = (float)pow2(-o.p);
+  o.scale = (float)pow2(o.s);
   o.rho2 = (float)(rr * rr * (1.0 - 0x1p-20));
   o.err = std::nextafter((float)err, INFINITY);
   o.lip = (float)(1.01 * lip);
@@ -280,7 +287,8 @@ struct Start {
   double hi, lo;  // |eps| of the class's samples, in units of 2^p: (lo, hi]
 };
 
-void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out) {
+void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out, int* stop) {
+  *stop = -1;
   const int f = std::max(1, st.fire - 3) - 1;
   const int last = od.xlen - 2;
   if (f < 1 || f >= last) return;
@@ -327,6 +335,7 @@ void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out) {
                         xm > 2.1 * dmax && xm + dmax < 1000.0;
       if (!good || n == last) {
         alive[i] = false;
+        if (*stop < 0 && !(xm > 2.1 * dmax)) *stop = n;
         if (n - 1 - f >= kMinSteps)
           make_record(prev, st.fire, n - 1, p, rho[i], prev_q[i], 0.0, out[i]);
         continue;
@@ -370,8 +379,9 @@ void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out) {
 
 }  // namespace
 
-void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int threads,
-                       std::vector<JumpRec>& out) {
+// The start jumps' records, and the orbit indexes at which classes ended near 0.
+static void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int threads,
+                              std::vector<JumpRec>& out, std::vector<int>& stops) {
   JumpRec none{};
   none.fire = -1;
   none.rho2 = -1.0f;
@@ -410,16 +420,18 @@ void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int threads
     above = r;
     i = lo;
   }
+  std::vector<int> stop(starts.size(), -1);
   std::atomic<size_t> next{0};
   auto work = [&] {
     for (size_t k; (k = next.fetch_add(1)) < starts.size();)
-      build_class(od, starts[k], p, &out[k * kJumpSubs]);
+      build_class(od, starts[k], p, &out[k * kJumpSubs], &stop[k]);
   };
   const size_t nt = std::min(starts.size(), (size_t)std::max(1, threads));
   std::vector<std::thread> pool;
   for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
   work();
   for (std::thread& t : pool) t.join();
+  stops = stop;
   // the classes in use first: the device stops at the first unused one, and
   // knows a class by its first record
   size_t at = 0;
@@ -435,13 +447,15 @@ void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int threads
   for (size_t k = at * kJumpSubs; k < out.size(); k++) out[k] = none;
 }
 
-void build_rebase_jumps(const OrbitData& od, double eps_m, int eps_e, std::vector<JumpRec>& out) {
-  constexpr int C = kRebaseClasses;
-  out.clear();
-  const int last = std::min(od.xlen - 2, kRebaseReach);
-  if (last < 2 * kMinSteps || !(eps_m >= 0.0) || !std::isfinite(eps_m)) return;
-  const double eps = eps_e < -1000 ? 0x1p-1000 : std::ldexp(eps_m, eps_e);
-  if (!(eps < 0x1p-16)) return;
+namespace {
+
+// The records of the chain that starts at orbit index s (X[s]) from delta = x,
+// x the whole of it; out: kChainClasses records.  stop: where its balls ended at
+// an element of the orbit near 0, most often (-1: nowhere).
+void build_chain(const OrbitData& od, int s, double eps, JumpRec* out, int* stop) {
+  constexpr int C = kChainClasses;
+  *stop = -1;
+  const int last = std::min(od.xlen - 2, s + kChainReach);
   // an order of eps weighs at most about 2^9 eps over the smallest ball's 2^-43
   // against the one before: as many as come to 2^-50 (below 2^-110 eps itself
   // is far under every bound)
@@ -453,40 +467,29 @@ void build_rebase_jumps(const OrbitData& od, double eps_m, int eps_e, std::vecto
   }
   Poly<B> u{};
   u.re[0][1] = 1.0;
-  // A sample's FP64 path need not rebase where the FP32 path does: it may hold
-  // the same point as Z' + delta' with |delta'| <= |w| and |Z'| <= 2 |w|, and
-  // then Z' runs along the orbit from Z'^2 + X[0], |Z'|^2 <= 4 |w|^2 <=
-  // 4 (|x| + (1 + |Gamma|) |eps|), which the class kHelper above this one
-  // holds (half of 16 rho0, rho0 the ball before the shifts; classes end below
-  // rho = 4 (1 + |Gamma|) eps).
-  constexpr int kHelper = 4;
   double rho[C], R[C], Q[C], P[C], E[C], S[C], H[C], T[C], order[B][C], power[2 * B];
   bool alive[C], open[C];
   power[0] = 1.0;
   for (int b = 1; b < 2 * B; b++) power[b] = power[b - 1] * eps;
   for (int i = 0; i < C; i++) {
-    rho[i] = std::exp2(-0.5 * kRebaseTop - i);
+    rho[i] = std::exp2(-0.5 * kChainTop - i);
     R[i] = P[i] = E[i] = 0.0;
-    // the FP64 path's rounding of its first step (delta = 0 * delta + ...)
+    // the FP64 path's rounding of the step that gave x
     Q[i] = 0x1p-49 * rho[i];
-    alive[i] = true;
-    open[i] = i >= kHelper;
+    alive[i] = open[i] = true;
   }
   double most = 0.0;
-  double gr = 0.0, gi = 0.0;  // Gamma: x = w^2 + (1 + Gamma) eps
-  JumpRec none{};
-  none.rho2 = -1.0f;
-  out.assign(C, none);
+  double gr = 0.0, gi = 0.0;  // Gamma: x = delta_s + Gamma eps
   Poly<B> prev = u;
   double prev_q[C] = {}, prev_rho[C] = {}, prev_g[2] = {};
   double a[B][D + 1] = {}, w[B][2 * D + 2];
   Shift shift;
-  for (int n = 0; n <= last; n++) {
+  int stops[C], nstops = 0;
+  for (int n = s; n <= last; n++) {
     const double xr = od.xhi[n].x, xi = od.xhi[n].y, xm = norm(xr, xi) * (1.0 + 0x1p-50);
     for (int b = 0; b < nb; b++)
       for (int k = 0; k < kTerms[b]; k++) a[b][k] = norm(u.re[b][k], u.im[b][k]);
     const bool end = n == last || !(a[0][D] < 0x1p900) || !(a[0][1] > 0.0);
-    bool any = false;
     // |delta|'s bounds: the polynomial's sums for the classes down to the first
     // that is nearly linear (`lin`).  From there on a smaller ball's nonlinear
     // part is at most the square of the ratio of the radii times that one's, an
@@ -519,24 +522,22 @@ void build_rebase_jumps(const OrbitData& od, double eps_m, int eps_e, std::vecto
       P[i] = a[0][1] * rho[i] + bend * t * t;
       E[i] = flat + slope * t;
     }
-    // a ball's own bound on |delta| holds while R is a small part of it
-    for (int i = 0; i < C; i++)
-      if (alive[i] && !(R[i] <= 0x1p-6 * P[i])) alive[i] = false;
+    bool any = false;
     for (int i = 0; i < C; i++) {
       if (!open[i]) continue;
-      const int h = i - kHelper;
+      // the FP64 path holds the sample at the same orbit index: it does not
+      // rebase while |delta| < |X| - |delta|, nor bail out below 1000
       const double d = P[i] + E[i] + R[i] + Q[i];
-      // |delta'| in the FP64 path's representation, |Z'| <= |X| + its helper's
-      const double d2 = alive[h] ? d + P[h] + E[h] + R[h] : INFINITY;
+      const bool near = n > s && !(xm > 2.1 * d);
       const bool good = alive[i] && !end && R[i] <= kTail * a[0][1] * rho[i] &&
-                        Q[i] <= 0x1p-20 * a[0][1] * rho[i] && xm > d + 1.1 * d2 &&
-                        xm + d2 < 1000.0;
+                        Q[i] <= 0x1p-20 * a[0][1] * rho[i] && !near && xm + d < 1000.0;
       if (good) {
         any = true;
         continue;
       }
       open[i] = false;
-      if (n - 1 < kMinSteps) continue;
+      if (near && alive[i] && n - s > 256) stops[nstops++] = n;
+      if (n - 1 - s < kMinSteps) continue;
       // the record's own Gamma, which takes the constant of order 1 out
       Poly<B> at = prev;
       double r = prev_rho[i], q = prev_q[i];
@@ -551,8 +552,8 @@ void build_rebase_jumps(const OrbitData& od, double eps_m, int eps_e, std::vecto
           shift.tr = shift.ti = 0.0;
         }
       }
-      if (!make_record(at, 0, n - 1, 0, r, q, nb > 1 ? eps : 0.0, out[i])) continue;
-      const double g1 = 1.0 + prev_g[0] + shift.tr, g2 = prev_g[1] + shift.ti;
+      if (!make_record(at, s, n - 1, 0, r, q, nb > 1 ? eps : 0.0, out[i])) continue;
+      const double g1 = prev_g[0] + shift.tr, g2 = prev_g[1] + shift.ti;
       Flt4& g = out[i].gamma;
       g.x = (float)g1;
       g.y = (float)(g1 - (double)g.x);
@@ -587,12 +588,10 @@ void build_rebase_jumps(const OrbitData& od, double eps_m, int eps_e, std::vecto
       const double h = i > lin ? H[lin] * t * t + T[lin] : H[i] + T[i];
       const double d = P[i] + E[i];
       R[i] = (2.0 * xm + 2.0 * d + R[i]) * R[i] + h;
-      const int hh = i - kHelper;
-      // the FP64 path's step at |Z'| <= |X| + d_h, |delta'| <= d + d_h
-      const double dh = hh >= 0 && alive[hh] ? P[hh] + E[hh] + R[hh] : 0.0;
+      // as build_class, with eps's own terms
       Q[i] = (2.0 * xm + 2.0 * d + Q[i]) * Q[i] + h +
-             0x1p-50 * (2.0 * xm + 3.0 * (d + dh)) * (d + dh) +
-             0x1p-50 * (1.5 * 2.0 * xm * d + 8.5 * d * d) + 0x1p-48 * eps;
+             0x1p-50 * (2.5 * 2.0 * xm * d + 9.5 * d * d) + 0x1p-48 * eps;
+      if (!(R[i] <= 0x1p-6 * P[i])) alive[i] = false;
     }
     if (nb == 1) continue;
     // Recentre (Shift) where the linear coefficient is the largest so far:
@@ -613,11 +612,55 @@ void build_rebase_jumps(const OrbitData& od, double eps_m, int eps_e, std::vecto
       Q[i] += r + shift.rounding(rho[i], eps);
       rho[i] -= shift.tm * eps;
       // (see Shift::dropped), and half of it in all
-      if (rho[i] < 0.5 * std::exp2(-0.5 * kRebaseTop - i) ||
-          rho[i] < 4.0 * (1.0 + norm(gr, gi)) * eps || shift.tm * eps > 0x1p-5 * rho[i])
+      if (rho[i] < 0.5 * std::exp2(-0.5 * kChainTop - i) || shift.tm * eps > 0x1p-5 * rho[i])
         alive[i] = false;
     }
   }
+  int count = 0;
+  for (int i = 0; i < nstops; i++) {
+    int c = 0;
+    for (int j = 0; j < nstops; j++) c += stops[j] == stops[i];
+    if (c > count) {
+      count = c;
+      *stop = stops[i];
+    }
+  }
+}
+
+}  // namespace
+
+void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t) {
+  JumpRec none{};
+  none.rho2 = -1.0f;
+  t.start_index.assign(kChains, -1);
+  std::vector<int> stops;
+  build_start_jumps(od, eps_m, eps_e, threads, t.start, stops);
+  t.chain.assign((size_t)kChains * kChainClasses, none);
+  if (od.xlen < 64 || !(eps_m >= 0.0) || !std::isfinite(eps_m)) return;
+  const double eps = eps_e < -1000 ? 0x1p-1000 : std::ldexp(eps_m, eps_e);
+  if (!(eps < 0x1p-16)) return;
+  // The chain from a rebase, and those from past the elements near 0 at which
+  // most start jumps (outermost samples first) and the rebase chain's end.
+  std::vector<int> from{0};
+  auto add = [&](int stop) {
+    if (stop >= 0 && stop + 1 + 4 * kMinSteps < od.xlen && (int)from.size() < kChains &&
+        std::find(from.begin(), from.end(), stop + 1) == from.end())
+      from.push_back(stop + 1);
+  };
+  for (size_t k = 0; k < stops.size() && k < 2; k++) add(stops[k]);
+  std::vector<std::thread> pool;
+  int stop[kChains];
+  for (size_t k = 1; k < from.size(); k++)
+    pool.emplace_back([&, k] {
+      build_chain(od, from[k], eps, &t.chain[k * kChainClasses], &stop[k]);
+    });
+  build_chain(od, 0, eps, &t.chain[0], &stop[0]);
+  for (std::thread& p : pool) p.join();
+  const size_t had = from.size();
+  add(stop[0]);
+  for (size_t k = had; k < from.size(); k++)
+    build_chain(od, from[k], eps, &t.chain[k * kChainClasses], &stop[k]);
+  for (size_t k = 0; k < from.size(); k++) t.start_index[k] = from[k];
 }
 
 }  // namespace nmg

@@ -302,7 +302,10 @@ __device__ __forceinline__ void persistent_loop(const DeviceView& v, const Rende
 // Producers append with k = atomicAdd(count, 1); list[k] = sample, and when a
 // producer warp has appended its last entry it fences and bumps `producers_done`.
 // Consumers claim entries [next, count) with a compare-and-swap on `next` (so
-// a claim never runs past the entries counted so far), read each entry until
+// a claim never runs past the entries counted so far; while producers run, only
+// as many as fill the warp's empty lanes: a warp instruction costs the FP64 pipe
+// the same with one lane as with 32, so the entries that trickle in have to
+// gather in few warps), read each entry until
 // it differs from kListSentinel (the list is filled with the sentinel before
 // the launch; the producer's store follows its atomicAdd at once), and stop
 // when every producer is done and every counted entry is claimed.  All waits
@@ -323,11 +326,12 @@ enum ClaimStatus { CLAIM_OK = 0, CLAIM_EMPTY = 1, CLAIM_BUSY = 2 };
 
 __device__ __forceinline__ int claim_entries(unsigned long long* next,
                                              const unsigned long long* count, unsigned want,
-                                             unsigned long long& base, unsigned& got) {
+                                             unsigned least, unsigned long long& base,
+                                             unsigned& got) {
   const unsigned long long end = *(const volatile unsigned long long*)count;
   for (int t = 0; t < 32; t++) {
     const unsigned long long c = *(volatile unsigned long long*)next;
-    if (c >= end) {
+    if (c >= end || end - c < least) {
       got = 0;
       return CLAIM_EMPTY;
     }
@@ -390,7 +394,8 @@ __device__ __forceinline__ void drain_loop(const Src& src, const RenderCtl& ctl,
         } else {
           done = *(const volatile unsigned long long*)producers_done >= producers;
           __threadfence();  // the count read below includes every finished producer's entries
-          status = claim_entries(ctl.next, ctl.count_ptr, __popc(need), base, got);
+          status = claim_entries(ctl.next, ctl.count_ptr, __popc(need),
+                                 done ? 1u : (unsigned)__popc(need), base, got);
         }
       }
       base = __shfl_sync(kFull, base, leader);

@@ -131,27 +131,28 @@ __device__ __forceinline__ void batch_iter_warp(const BatchGroup& grp, const FeP
       }
     }
     if (!__any_sync(kFull, active)) break;
-    if (active) {
-      FeResult res;
-      const DeviceView& v = grp.views[f];
-      // the arithmetic of the frame rendered alone (render_fe32.cu): t = 2Z +
-      // delta unnormalised on frames inside the FP64 range
+    FeResult res;
+    const DeviceView& v = grp.views[f];
+    // the arithmetic of the frame rendered alone (render_fe32.cu): t = 2Z +
+    // delta unnormalised on frames inside the FP64 range
+    const bool done = fe_round(v, st, active, chunk, [&](int n) {
       FeTrap* trap = v.trap ? v.trap + (g - grp.offsets[f]) : nullptr;
-      if (fe_raw_t(v) ? fe_advance<false, true>(v, st, chunk, res, executed, rebases, trap)
-                      : fe_advance<false, false>(v, st, chunk, res, executed, rebases, trap)) {
-        int r = 0, c = 0;
-        sample_rc(v, g - grp.offsets[f], r, c);
-        log_cost(v, r, c, executed - exec0, 1);
-        if (st.certified) {
-          const float s = fe_smoothing(v, res);
-          store_sample(v, r, c, EscapeValue{res.it, s}, s);
-        } else {  // rendered by the FP64 kernel
-          const unsigned long long k = atomicAdd(ctl.rework_n, 1ull);
-          ctl.rework[k] = g;
-        }
-        finished++;
-        active = false;
+      return fe_raw_t(v) ? fe_advance<false, true>(v, st, n, res, executed, rebases, trap)
+                         : fe_advance<false, false>(v, st, n, res, executed, rebases, trap);
+    });
+    if (done) {
+      int r = 0, c = 0;
+      sample_rc(v, g - grp.offsets[f], r, c);
+      log_cost(v, r, c, executed - exec0, 1);
+      if (st.certified) {
+        const float s = fe_smoothing(v, res);
+        store_sample(v, r, c, EscapeValue{res.it, s}, s);
+      } else {  // rendered by the FP64 kernel
+        const unsigned long long k = atomicAdd(ctl.rework_n, 1ull);
+        ctl.rework[k] = g;
       }
+      finished++;
+      active = false;
     }
   }
   for (int o = 16; o > 0; o >>= 1) {

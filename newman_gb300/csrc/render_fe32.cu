@@ -53,6 +53,7 @@ struct FeJob {
                                                unsigned long long& executed,
                                                unsigned long long& rebases) {
     FeResult res;
+    if (fe_may_jump(v, st)) fe_chain_jump(v, st);
     if (!fe_advance<false, kRawT>(v, st, n, res, executed, rebases)) return false;
     const float s = fe_smoothing(v, res);
     sm = s;
@@ -163,23 +164,24 @@ __device__ __forceinline__ void fe_iter_warp(const DeviceView& v, const FePassBu
       }
     }
     if (!__any_sync(kFull, active)) break;
-    if (active) {
-      FeResult res;
-      if (fe_advance<kStaged, kRawT>(v, st, chunk, res, executed, rebases,
-                              v.trap ? v.trap + sid : nullptr)) {
-        int r = 0, c = 0;
-        sample_rc(v, sid, r, c);
-        if (st.certified) {
-          const float s = fe_smoothing(v, res);
-          store_sample(v, r, c, EscapeValue{res.it, s}, s);
-        } else {  // rendered by the FP64 kernel
-          const unsigned long long k = atomicAdd(ctl.rework_n, 1ull);
-          ctl.rework[k] = sid;
-        }
-        log_cost(v, r, c, executed - exec0, 1);
-        finished++;
-        active = false;
+    FeResult res;
+    const bool done = fe_round(v, st, active, chunk, [&](int n) {
+      return fe_advance<kStaged, kRawT>(v, st, n, res, executed, rebases,
+                                        v.trap ? v.trap + sid : nullptr);
+    });
+    if (done) {
+      int r = 0, c = 0;
+      sample_rc(v, sid, r, c);
+      if (st.certified) {
+        const float s = fe_smoothing(v, res);
+        store_sample(v, r, c, EscapeValue{res.it, s}, s);
+      } else {  // rendered by the FP64 kernel
+        const unsigned long long k = atomicAdd(ctl.rework_n, 1ull);
+        ctl.rework[k] = sid;
       }
+      log_cost(v, r, c, executed - exec0, 1);
+      finished++;
+      active = false;
     }
   }
   for (int o = 16; o > 0; o >>= 1) {

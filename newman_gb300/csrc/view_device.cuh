@@ -71,23 +71,32 @@ constexpr int32_t kTfeInf = 0x7fffffff, kTfeZero = -0x7fffffff;
 // included.
 constexpr int kJumpDegree = 16;
 constexpr int kJumpExact = 7;     // terms in float-float; the rest in FP32
-constexpr int kJumpOrders = 5;    // orders of eps (rebase jumps), with terms
+// Orders of eps (chain jumps), with terms; order 1's constant is 0 but where a
+// record could not be centred on it, and its first kEpsExact terms are in
+// float-float.
+constexpr int kJumpOrders = 5;
+constexpr int kEpsExact = 5;
 constexpr int kJumpEps1 = 8, kJumpEps2 = 5, kJumpEps3 = 3, kJumpEps4 = 2;
 constexpr int kJumpClasses = 12;  // series stop indexes
 constexpr int kJumpSubs = 7;      // radii of each
-constexpr int kRebaseClasses = 36;
-constexpr int kRebaseTop = 16;    // class i: |x|^2 < 2^-(kRebaseTop + 2 i)
+constexpr int kChains = 3;        // orbit indexes that chain jumps start from
+constexpr int kChainClasses = 36;
+constexpr int kChainTop = 16;     // class i: |x|^2 < 2^-(kChainTop + 2 i)
 struct Flt2 {
   float x, y;
 };
 struct alignas(16) JumpRec {
   int32_t fire, n, p, s;
   float rho2, err, lip, lip2;  // bounds of |d delta_n / dx| and of half its second
-  Flt4 gamma;          // 1 + Gamma (rebase jumps)
+  float unit, scale;   // 2^-p, 2^s (chain jumps)
+  int32_t pad_[2];
+  Flt4 gamma;          // Gamma (chain jumps)
   Flt4 b[kJumpExact];  // {re.h, re.l, im.h, im.l}, as gamma
   Flt2 c[kJumpDegree - kJumpExact];
+  Flt2 d[kJumpDegree];  // the derivative's coefficients (k + 1) u_k+1 (chain jumps)
   // of (2^32 eps)^1 .. (2^32 eps)^4
   Flt2 q1[kJumpEps1], q2[kJumpEps2], q3[kJumpEps3], q4[kJumpEps4];
+  Flt2 q1l[kEpsExact];  // q1's low words
 };
 
 enum CardioidMode : int32_t {
@@ -144,8 +153,10 @@ struct DeviceView {
   const CFFE* sa_b32;
   const CFFE* sa_c32;
   const TFE* sa_min32;     // [xlen]
-  const JumpRec* jump;     // [kJumpClasses * kJumpSubs], then [kRebaseClasses]; or null
-  float jump_w2;           // rebases with |w|^2 below it may jump (0: none)
+  const JumpRec* jump;     // [kJumpClasses * kJumpSubs], then [kChains * kChainClasses];
+                           // or null
+  int32_t jump_from[kChains];  // orbit indexes j (of z) of the chains' starts; -1: none
+  float jump_x2;           // starts with |delta|^2 below it may jump (0: none)
 
   // the reference-exact path: values in the view's arbitrary precision as
   // records of mp_limbs limbs (mpf_fixed.cuh; word 0: exponent << 32 | sign)

@@ -38,8 +38,9 @@ int main(int argc, char** argv) {
   for (const RFE& y : ei) my = std::max(my, fabsl(ldexpl(y.m, y.e)));
   const LD m = sqrtl(mx * mx + my * my);
   const int e = ilogbl(m);
-  std::vector<JumpRec> recs;
-  build_start_jumps(od, (double)ldexpl(m, -e) * (1.0 + 0x1p-40), e, 4, recs);
+  JumpTables tables;
+  build_jumps(od, (double)ldexpl(m, -e) * (1.0 + 0x1p-40), e, 4, tables);
+  const std::vector<JumpRec>& recs = tables.start;
   // to 53 bits: the FP64 path's rounding, with its unbounded exponent
   auto r53 = [](LD x) {
     if (x == 0) return x;
@@ -101,36 +102,34 @@ int main(int argc, char** argv) {
     worst = std::max(worst, std::max(e1, e2) / bound);
     if (event || !(e1 <= bound) || !(e2 <= bound)) bad++;
   }
-  // rebase jumps: w on a circle of the ball's size, both with the FP64 path at
-  // the same index and with it left at (Z', w - Z') as after a near return it
-  // did not rebase at
-  std::vector<JumpRec> rb;
-  build_rebase_jumps(od, (double)ldexpl(m, -e) * (1.0 + 0x1p-40), e, rb);
+  // chain jumps: delta on a circle of the ball's size at each chain's start
   long rj = 0, rbad = 0;
   LD rworst = 0, rsteps = 0;
   std::uniform_real_distribution<double> U(0.0, 1.0);
   auto X = [&](int n) { return CL((LD)od.xhi[n].x + od.xlo[n].x, (LD)od.xhi[n].y + od.xlo[n].y); };
-  for (int s = 0; s < samples && !rb.empty(); s++) {
+  for (int s = 0; s < samples; s++) {
+    const int chain = s % kChains, from = tables.start_index[chain];
+    if (from < 0) continue;
+    const JumpRec* rb = &tables.chain[(size_t)chain * kChainClasses];
     const RFE& a = er[g() % er.size()];
     const RFE& b = ei[g() % ei.size()];
     const CL eps(ldexpl(a.m, a.e), ldexpl(b.m, b.e));
-    const LD wm = exp2l(-0.25L * (kRebaseTop + 2 * kRebaseClasses * U(g))), ph = 6.2831853L * U(g);
-    const CL w(r53(wm * cosl(ph)), r53(wm * sinl(ph)));
-    int i = (-(ilogbl(std::norm(w * w + eps)) + 1) - kRebaseTop) >> 1;
+    const LD dm = exp2l(-0.5L * (kChainTop + 2 * kChainClasses * U(g))), ph = 6.2831853L * U(g);
+    const CL d0(r53(dm * cosl(ph)), r53(dm * sinl(ph)));
+    int i = (-(ilogbl(std::norm(d0)) + 1) - kChainTop) >> 1;
     const JumpRec* use = nullptr;
     CL x = 0;
     for (int t = 0; t < 3 && !use; t++, i--) {
-      if (i < 0 || i >= kRebaseClasses || !(rb[i].rho2 > 0)) continue;
+      if (i < 0 || i >= kChainClasses || !(rb[i].rho2 > 0)) continue;
       const Flt4 g = rb[i].gamma;
-      x = w * w + CL((LD)g.x + g.y, (LD)g.z + g.w) * eps;
+      x = d0 + CL((LD)g.x + g.y, (LD)g.z + g.w) * eps;
       if (ldexpl(std::norm(x), -2 * rb[i].p) <= rb[i].rho2) use = &rb[i];
     }
     if (!use) continue;
     rj++;
     const int n = use->n;
-    rsteps += n + 1;
-    CL d = w * w + eps;
-    for (int k = 0; k < n; k++) d = (X(k) + X(k) + d) * d + eps;
+    if (use->fire != from) rbad++;
+    rsteps += n - from;
     // the polynomial
     const CL y(ldexpl(x.real(), -use->p), ldexpl(x.imag(), -use->p));
     CL p = 0, q = 0;
@@ -141,50 +140,41 @@ int main(int argc, char** argv) {
     const int len[4] = {kJumpEps4, kJumpEps3, kJumpEps2, kJumpEps1};
     for (int o = 0; o < 4; o++) {
       CL t = 0;
-      for (int k = len[o] - 1; k >= 0; k--) t = t * y + CL(tab[o][k].x, tab[o][k].y);
+      for (int k = len[o] - 1; k >= 0; k--) {
+        t = t * y + CL(tab[o][k].x, tab[o][k].y);
+        if (o == 3 && k < kEpsExact) t += CL(use->q1l[k].x, use->q1l[k].y);
+      }
       q = (q + t) * 0x1p32L * eps;
     }
     p = p * y + q;
-    const LD e1 = std::abs(p - CL(ldexpl(d.real(), -use->s), ldexpl(d.imag(), -use->s)));
-    rworst = std::max(rworst, e1 / use->err);
-    bool ok = e1 <= use->err;
-    // the FP64 path from (Z', delta'): Z' an orbit element or 0
-    for (int t = 0; t < 2 && ok; t++) {
-      int j = 0;
-      LD dr = w.real(), di = w.imag();
-      if (t == 1) {  // an orbit element near enough to w
-        j = -1;
-        for (int k = 1; k < od.xlen - n - 2; k++)
-          if (std::abs(X(k - 1)) <= 2 * wm && std::abs(w - X(k - 1)) <= wm) { j = k; break; }
-        if (j < 0) break;
-        dr = r53(w.real() - od.xhi[j - 1].x);
-        di = r53(w.imag() - od.xhi[j - 1].y);
-      }
-      CL td(dr, di);  // the exact orbit of its start point, in its representation
-      bool event = false;
-      for (int k = 0; k <= n; k++, j++) {
-        const LD zr = j ? od.xhi[j - 1].x : 0.0, zi = j ? od.xhi[j - 1].y : 0.0;
-        const LD tr = r53(2 * zr + dr), ti = r53(2 * zi + di);
-        const LD nre = r53(r53(r53(tr * dr) - r53(ti * di)) + eps.real());
-        const LD nim = r53(r53(r53(tr * di) + r53(ti * dr)) + eps.imag());
-        dr = nre;
-        di = nim;
-        const CL xe = j ? X(j - 1) : CL(0);
-        td = (xe + xe + td) * td + eps;
-        const LD yr = od.xhi[j].x + dr, yi = od.xhi[j].y + di;
-        if (yr * yr + yi * yi <= dr * dr + di * di || yr * yr + yi * yi > 1048576.0L) event = true;
-      }
-      const LD e2 = ldexpl(std::abs(CL(dr, di) - td), -use->s);
-      rworst = std::max(rworst, e2 / use->err);
-      ok = e2 <= use->err && !event;
+    // the exact orbit, and the FP64 path's steps
+    CL d = d0;
+    LD dr = d0.real(), di = d0.imag();
+    bool event = false;
+    for (int k = from; k < n; k++) {
+      d = (X(k) + X(k) + d) * d + eps;
+      const LD tr = r53(2 * (LD)od.xhi[k].x + dr), ti = r53(2 * (LD)od.xhi[k].y + di);
+      const LD nre = r53(r53(r53(tr * dr) - r53(ti * di)) + eps.real());
+      const LD nim = r53(r53(r53(tr * di) + r53(ti * dr)) + eps.imag());
+      dr = nre;
+      di = nim;
+      const LD yr = od.xhi[k + 1].x + dr, yi = od.xhi[k + 1].y + di;
+      if (yr * yr + yi * yi <= dr * dr + di * di || yr * yr + yi * yi > 1048576.0L) event = true;
     }
-    if (!ok) rbad++;
+    const LD e1 = std::abs(p - CL(ldexpl(d.real(), -use->s), ldexpl(d.imag(), -use->s)));
+    const LD e2 = std::abs(p - CL(ldexpl(dr, -use->s), ldexpl(di, -use->s)));
+    rworst = std::max(rworst, std::max(e1, e2) / use->err);
+    if (event || !(e1 <= use->err) || !(e2 <= use->err)) rbad++;
   }
   std::printf("%ld %ld %.1f %.4f\n", rj, rbad, (double)(rsteps / std::max(1L, rj)), (double)rworst);
   if (std::getenv("JUMP_RECORDS"))
-    for (size_t i = 0; i < rb.size(); i++)
-      std::printf("class %zu n %d p %d s %d err 2^%.1f lip %.2f q0 %.2g rho %.2f\n", i, rb[i].n, rb[i].p, rb[i].s,
-                  std::log2(rb[i].err), rb[i].lip, rb[i].q1[0].x, std::sqrt(std::max(0.f, rb[i].rho2)));
+    for (size_t i = 0; i < tables.chain.size(); i++) {
+      const JumpRec& r = tables.chain[i];
+      if (r.rho2 > 0)
+        std::printf("chain %d class %zu n %d p %d s %d err 2^%.1f q0 %.2g rho %.2f\n", r.fire,
+                    i % kChainClasses, r.n, r.p, r.s, std::log2(r.err), r.q1[0].x,
+                    std::sqrt(r.rho2));
+    }
   if (rbad) bad += rbad;
   std::printf("%d %ld %ld %.1f %.4f\n", samples, jumped, bad, (double)(steps / std::max(1L, jumped)),
               (double)worst);
