@@ -460,11 +460,11 @@ __device__ __forceinline__ FF ff_norm2(FF x, FF y) {
 
 // The bailout test on Y = Z + delta (unscaled, float-float).  Returns true
 // when |Y|^2 > 2^20; clears `certified` when the error bound `yerr` on |Y|
-// reaches across 1024, or (kSmooth) when an escaped sample's exceeds |Y| / 4: the
-// smoothing term moves by up to 0.21 of the relative error of |Y|, and a bound of
-// |Y| itself let it differ from the FP64 path's by 4e-4 (the 3840x2160 view at
-// 1e-300, one sample in 3 million) where this lets it by 2e-4, for 7 % more
-// reworked samples.
+// reaches across 1024, or (kSmooth) when an escaped sample's exceeds |Y| / 16:
+// the smoothing term moves by up to 0.21 of the relative error of |Y|.  With a
+// bound of |Y| itself it differed from the FP64 path's by up to 4e-4 (the
+// 3840x2160 view at 1e-300), with |Y| / 4 by 3e-4, with |Y| / 16 by 1e-4 (as much
+// as before the jumps); the last costs 15 % more reworked samples than the first.
 template <bool kSmooth>
 __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& certified,
                                                FF& r2) {
@@ -473,7 +473,7 @@ __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& c
   // | |Y| - 1024 | <= 2 yerr  <=>  | |Y|^2 - 2^20 | <= (2048 + 2 yerr) 2 yerr
   if (fabsf(d) <= up_fma(up_fma(2.0f, yerr, 2048.0f), up_mul(2.0f, yerr), up_mul(0x1p-40f, r2.h)))
     certified = false;
-  if (kSmooth && d > 0.0f && up_mul(16.0f * yerr, yerr) > r2.h) certified = false;
+  if (kSmooth && d > 0.0f && up_mul(256.0f * yerr, yerr) > r2.h) certified = false;
   return d > 0.0f;
 }
 

@@ -194,6 +194,11 @@ __device__ __forceinline__ bool pool_exchange(SamplePool<typename Job::State>* p
   return leave;
 }
 
+// A warp takes new samples once this many lanes are empty (or all work has to
+// start): a job's start (the series front in FP64) costs the warp the same for
+// one lane as for eight, some 100 FP64 instructions.
+constexpr int kRefillLanes = 8;
+
 template <class Job, class Src>
 __device__ __forceinline__ void sample_loop(const Src& src, const RenderCtl& ctl, int chunk,
                                             SamplePool<typename Job::State>* pool = nullptr) {
@@ -216,7 +221,7 @@ __device__ __forceinline__ void sample_loop(const Src& src, const RenderCtl& ctl
     // the cardioid, so repeat until every lane is busy or the work is gone).
     for (;;) {
       const unsigned need = __ballot_sync(kFull, !active && !exhausted);
-      if (!need) break;
+      if (__popc(need) < kRefillLanes && (!need || __any_sync(kFull, active))) break;
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
       if (lane == leader) {
@@ -380,8 +385,8 @@ __device__ __forceinline__ void drain_loop(const Src& src, const RenderCtl& ctl,
   pool_enter(pool);
   for (;;) {
     const unsigned need = __ballot_sync(kFull, !active);
-    bool dry = need != 0;  // empty lanes the list could not fill
-    if (need && !closed) {
+    bool dry = __popc(need) >= kRefillLanes;  // empty lanes the list could not fill
+    if (__popc(need) >= kRefillLanes && !closed) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
       unsigned got = 0;

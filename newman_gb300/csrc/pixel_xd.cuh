@@ -168,11 +168,18 @@ NM_HD bool delta_guarded_steps(const DeviceView& v, DeltaState& st, int steps, E
     const Dbl2 zn = orbit_z<kStaged>(v, j < zlast ? j + 1 : zlast);  // loaded before the step's arithmetic
     const double tr = add_(twice_(z.x), dr);
     const double ti = add_(twice_(z.y), di);
-    const double nre = add_(sub_(mul_(tr, dr), mul_(ti, di)), st.er);
-    const double nim = add_(add_(mul_(tr, di), mul_(ti, dr)), st.ei);
+    double nre = sub_(mul_(tr, dr), mul_(ti, di));
+    double nim = add_(mul_(tr, di), mul_(ti, dr));
+    // eps, where it is not below half an ulp (on a view at 1e-300 it is from a
+    // few steps on: 2 of 10 FP64 operations)
+    if (!(absorbed(nre, st.er) && absorbed(nim, st.ei))) {
+      nre = add_(nre, st.er);
+      nim = add_(nim, st.ei);
+    }
     // Y = Z + delta only where the tests need it (delta_steps); a Y that is
     // not formed feeds nothing, so only the formed values are guarded
-    const bool need_y = j + 1 == zlast || !no_event_before_y(zn, nre, nim);
+    const bool need_y =
+        j + 1 == zlast || !(no_event_before_y(zn, nre, nim) || no_event_by_estimate(zn, nre, nim));
     double yr = 0.0, yi = 0.0;
     if (need_y) {
       yr = add_(zn.x, nre);
