@@ -460,11 +460,12 @@ __device__ __forceinline__ FF ff_norm2(FF x, FF y) {
 
 // The bailout test on Y = Z + delta (unscaled, float-float).  Returns true
 // when |Y|^2 > 2^20; clears `certified` when the error bound `yerr` on |Y|
-// reaches across 1024, or (kSmooth) when an escaped sample's exceeds |Y| / 16:
+// reaches across 1024, or (kSmooth) when an escaped sample's exceeds |Y| / 8:
 // the smoothing term moves by up to 0.21 of the relative error of |Y|.  With a
 // bound of |Y| itself it differed from the FP64 path's by up to 4e-4 (the
-// 3840x2160 view at 1e-300), with |Y| / 4 by 3e-4, with |Y| / 16 by 1e-4 (as much
-// as before the jumps); the last costs 15 % more reworked samples than the first.
+// 3840x2160 view at 1e-300; 1e-4 before the jumps), with |Y| / 8 by 2e-4, with
+// |Y| / 16 by 1e-4; the last costs 20 % more reworked samples than the first
+// (66 -> 75 ms a frame there), the second 9 %.
 template <bool kSmooth>
 __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& certified,
                                                FF& r2) {
@@ -473,7 +474,7 @@ __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& c
   // | |Y| - 1024 | <= 2 yerr  <=>  | |Y|^2 - 2^20 | <= (2048 + 2 yerr) 2 yerr
   if (fabsf(d) <= up_fma(up_fma(2.0f, yerr, 2048.0f), up_mul(2.0f, yerr), up_mul(0x1p-40f, r2.h)))
     certified = false;
-  if (kSmooth && d > 0.0f && up_mul(256.0f * yerr, yerr) > r2.h) certified = false;
+  if (kSmooth && d > 0.0f && up_mul(64.0f * yerr, yerr) > r2.h) certified = false;
   return d > 0.0f;
 }
 
@@ -956,7 +957,7 @@ __device__ __forceinline__ bool fe_may_jump(const DeviceView& v, const FeState& 
 // step the chunk in one go (their trapping test runs once a call).  Every lane
 // of the warp calls it; true, per lane, when its sample is finished.
 constexpr int kFeBurst = 16;
-constexpr int kFeIdle = 10;
+constexpr int kFeIdle = 12;
 template <class Advance>
 __device__ __forceinline__ bool fe_round(const DeviceView& v, FeState& st, bool active, int chunk,
                                          Advance advance) {

@@ -13,6 +13,7 @@ namespace nmg {
 
 struct HwJob {
   using State = HwState;
+  static constexpr int kRefill = 1;
   static constexpr bool kCertifies = false;
   static constexpr int kCostWeight = kCostFp64Step;
   static __device__ __forceinline__ bool certified(const State&) { return true; }
@@ -49,6 +50,7 @@ struct Delta64JobT {
     };
     int32_t xd;  // 1: in the unbounded-exponent form
   };
+  static constexpr int kRefill = 4;
   static constexpr bool kCertifies = false;
   static constexpr int kCostWeight = kCostFp64Step;
   static __device__ __forceinline__ bool certified(const State&) { return true; }
@@ -102,6 +104,7 @@ struct Fp64AnyJobT {
     HwJob::State hw;
     typename Delta64JobT<kStaged>::State d;
   };
+  static constexpr int kRefill = 4;
   static constexpr bool kCertifies = false;
   static constexpr int kCostWeight = kCostFp64Step;
   static __device__ __forceinline__ bool certified(const State&) { return true; }

@@ -194,11 +194,12 @@ __device__ __forceinline__ bool pool_exchange(SamplePool<typename Job::State>* p
   return leave;
 }
 
-// A warp takes new samples once this many lanes are empty (or all work has to
-// start): a job's start (the series front in FP64) costs the warp the same for
-// one lane as for eight, some 100 FP64 instructions.
-constexpr int kRefillLanes = 8;
-
+// A warp takes new samples once Job::kRefill lanes are empty (or all work has to
+// start): the series front in FP64 costs the warp the same for one lane as for
+// four, some 100 FP64 instructions (FE32 rework of the 1920x1080x16 view at
+// 1e-12 with 1, 4 and 8 lanes: 117, 86, 86 ms for the frame; the FP64 path there,
+// 961x541x4: 84, 81, 80 ms).  A double-loop start is cheap and its samples can be
+// short: one lane (640x480 view of width 3: 0.71, 0.73, 0.77 ms).
 template <class Job, class Src>
 __device__ __forceinline__ void sample_loop(const Src& src, const RenderCtl& ctl, int chunk,
                                             SamplePool<typename Job::State>* pool = nullptr) {
@@ -221,7 +222,7 @@ __device__ __forceinline__ void sample_loop(const Src& src, const RenderCtl& ctl
     // the cardioid, so repeat until every lane is busy or the work is gone).
     for (;;) {
       const unsigned need = __ballot_sync(kFull, !active && !exhausted);
-      if (__popc(need) < kRefillLanes && (!need || __any_sync(kFull, active))) break;
+      if (__popc(need) < Job::kRefill && (!need || __any_sync(kFull, active))) break;
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
       if (lane == leader) {
@@ -385,8 +386,8 @@ __device__ __forceinline__ void drain_loop(const Src& src, const RenderCtl& ctl,
   pool_enter(pool);
   for (;;) {
     const unsigned need = __ballot_sync(kFull, !active);
-    bool dry = __popc(need) >= kRefillLanes;  // empty lanes the list could not fill
-    if (__popc(need) >= kRefillLanes && !closed) {
+    bool dry = __popc(need) >= Job::kRefill;  // empty lanes the list could not fill
+    if (__popc(need) >= Job::kRefill && !closed) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
       unsigned got = 0;

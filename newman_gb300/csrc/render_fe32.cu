@@ -41,6 +41,7 @@ namespace {
 template <bool kRawT>
 struct FeJob {
   using State = FeState;
+  static constexpr int kRefill = 1;
   static constexpr bool kCertifies = true;
   static constexpr int kCostWeight = 1;
   static __device__ __forceinline__ bool init(const DeviceView& v, int r, int c, State& st,
