@@ -833,7 +833,7 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
   long long need_blocks = (max_useful + warps_per_block - 1) / warps_per_block;
   if (blocks > need_blocks) blocks = (int)need_blocks;
   if (blocks < 1) blocks = 1;
-  int chunk = h->chunk;
+  int chunk = h->fp64_chunk(kind == nmg::KERNEL_HW || kind == nmg::KERNEL_HW_MP);
   if (kind == nmg::KERNEL_FE32)  // the FE32 kernel renormalises per chunk
     chunk = h->renorm > 0 ? h->renorm : (v.sa_fe ? 32 : 64);
   NM_CUDA(cudaEventRecord(h->ev[0], s));
@@ -853,7 +853,7 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
       o.rework = rework_ctl(h, ctl);
       o.fe_warps_done = h->d_scratch.p + kFeWarpsDone;
       o.timeouts = h->d_scratch.p + kStatsMain + nmg::STAT_WAIT_TIMEOUTS;
-      o.chunk = h->chunk;
+      o.chunk = h->fp64_chunk(false);
     }
     // Staging the orbit's first entries: measured on the 3840x2160 view at
     // width 1e-300 (floatexp series) 32.3 -> 31.4 ms with 1024 entries (31.7
@@ -877,7 +877,7 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
     // an overlapped iteration pass: only the entries it left unclaimed).
     const nmg::RenderCtl re = rework_ctl(h, ctl);
     int rblocks = h->blocks > 0 ? h->blocks : nmg::persistent_blocks(nmg::KERNEL_REWORK, h->device);
-    NM_CUDA(nmg::launch_render(nmg::KERNEL_REWORK, v, re, s, rblocks, h->chunk));
+    NM_CUDA(nmg::launch_render(nmg::KERNEL_REWORK, v, re, s, rblocks, h->fp64_chunk(false)));
     NM_CUDA(cudaEventRecord(h->ev[2], s));
   }
   return NM_OK;
@@ -904,7 +904,8 @@ int nm_synchronize(nm_handle* h) {
       const nmg::RenderCtl re = rework_ctl(h, main);
       NM_CUDA(cudaMemsetAsync(h->d_scratch.p + kNextRework, 0, 8, s));
       NM_CUDA(nmg::launch_render(nmg::KERNEL_REWORK, h->last_view, re, s,
-                                 nmg::persistent_blocks(nmg::KERNEL_REWORK, h->device), h->chunk));
+                                 nmg::persistent_blocks(nmg::KERNEL_REWORK, h->device),
+                                 h->fp64_chunk(false)));
       NM_CUDA(cudaStreamSynchronize(s));
     }
   }
