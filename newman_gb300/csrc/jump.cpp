@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <system_error>
 #include <thread>
 
 namespace nmg {
@@ -428,7 +429,10 @@ static void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int 
   };
   const size_t nt = std::min(starts.size(), (size_t)std::max(1, threads));
   std::vector<std::thread> pool;
-  for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
+  try {
+    for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
+  } catch (const std::system_error&) {  // no more threads: with those there are
+  }
   work();
   for (std::thread& t : pool) t.join();
   stops = stop;
@@ -650,10 +654,14 @@ void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, Jump
   for (size_t k = 0; k < stops.size() && k < 2; k++) add(stops[k]);
   std::vector<std::thread> pool;
   int stop[kChains];
-  for (size_t k = 1; k < from.size(); k++)
-    pool.emplace_back([&, k] {
-      build_chain(od, from[k], eps, &t.chain[k * kChainClasses], &stop[k]);
-    });
+  for (size_t k = 1; k < from.size(); k++) {
+    auto one = [&, k] { build_chain(od, from[k], eps, &t.chain[k * kChainClasses], &stop[k]); };
+    try {
+      pool.emplace_back(one);
+    } catch (const std::system_error&) {
+      one();
+    }
+  }
   build_chain(od, 0, eps, &t.chain[0], &stop[0]);
   for (std::thread& p : pool) p.join();
   const size_t had = from.size();

@@ -54,7 +54,7 @@ struct MpJob {
     Mpfx<P> yr, yi, y0r, y0i;
     int32_t i;
   };
-  static constexpr int kRefill = 4;
+  static constexpr int kRefill = 1;
   static constexpr bool kCertifies = false;
   static constexpr int kCostWeight = 1;
   static __device__ __forceinline__ bool certified(const State&) { return true; }
