@@ -70,8 +70,7 @@ enum nm_option {
   NM_OPT_KEEP_SMOOTH64 = 3, /* 1: also keep the unrounded double smoothing */
   NM_OPT_THREADS = 4,     /* host threads for the probe search (0 = all) */
   NM_OPT_BLOCKS = 5,      /* persistent blocks (0 = fill the GPU) */
-  NM_OPT_RENORM = 6,      /* FE32: steps between exponent renormalisations (0: 64,
-                             32 on views below the double range) */
+  NM_OPT_RENORM = 6,      /* FE32: steps between exponent renormalisations (0: 64) */
   NM_OPT_FE32_SINGLE_PASS = 7, /* FE32 in one persistent kernel (default: three passes) */
   NM_OPT_REFERENCE = 8,   /* reference orbit: 0 the reference's probe search
                              (findProbe, mandelbrot.cpp:73-95), 1 the view center */
@@ -83,8 +82,7 @@ enum nm_option {
                                   (2, 4 or 6; 0 = 4 with double-loop frames, else 2) */
   NM_OPT_ORBIT_STAGE = 13,  /* FE32 iteration pass: the first n (0..3072) reference-orbit entries
                                copied into each block's shared memory by the TMA unit, where
-                               every rebased sample restarts (0: none; -1, the default: 1024 on
-                               views whose series leaves the double range, else none) */
+                               every rebased sample restarts (0, and -1, the default: none) */
   NM_OPT_L2_WINDOW = 14,    /* FE32 iteration pass: 1 runs it with a persisting L2 access-policy
                                window over the reference orbit (the process's L2 set-aside is
                                raised to the orbit's size, within the device's limit) */

@@ -44,10 +44,6 @@ constexpr unsigned long kDoubleLoopOrbitBits = 256;
 // path renders with the double loop directly -- the same escape counts.
 constexpr double kDoubleLoopFe32MinStep = 0x1p-33;
 
-// Orbit entries staged in shared memory by default on views whose series
-// leaves the double range (NM_OPT_ORBIT_STAGE -1).
-constexpr int kAutoOrbitStage = 1024;
-
 // An upper bound on |c|_1 over the samples of the view (their coordinates as
 // the double loop takes them), as a float.
 float coord_abs_bound(const nm_handle* h) {
@@ -835,7 +831,7 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
   if (blocks < 1) blocks = 1;
   int chunk = h->fp64_chunk(kind == nmg::KERNEL_HW || kind == nmg::KERNEL_HW_MP);
   if (kind == nmg::KERNEL_FE32)  // the FE32 kernel renormalises per chunk
-    chunk = h->renorm > 0 ? h->renorm : (v.sa_fe ? 32 : 64);
+    chunk = h->renorm > 0 ? h->renorm : 64;
   NM_CUDA(cudaEventRecord(h->ev[0], s));
   h->timed_iter = false;
   if (kind == nmg::KERNEL_FE32 && !h->fe_single_pass) {
@@ -855,11 +851,12 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
       o.timeouts = h->d_scratch.p + kStatsMain + nmg::STAT_WAIT_TIMEOUTS;
       o.chunk = h->fp64_chunk(false);
     }
-    // Staging the orbit's first entries: measured on the 3840x2160 view at
-    // width 1e-300 (floatexp series) 32.3 -> 31.4 ms with 1024 entries (31.7
-    // with 2048); on the 1920x1080x16 view at 1e-12 no change with 1024 and
-    // 12 % slower with 2048 (3 blocks an SM instead of 4).
-    const int stage = h->z_stage >= 0 ? h->z_stage : (v.sa_fe ? kAutoOrbitStage : 0);
+    // No orbit entries staged unless asked for: a rebased sample leaves the first
+    // entries by a jump, and the shared memory is better left to the L1 (3840x2160
+    // at width 1e-300 with 0, 512 and 1024 entries 63.0, 64.7, 64.8 ms; at 1e-330
+    // 161, 166, 165; 2x2 samples at 1e-412 1,086, 1,110, 1,127; the 1920x1080x16 view
+    // at 1e-12 with 0 and 1024 84.5, 86.2).
+    const int stage = h->z_stage >= 0 ? h->z_stage : 0;
     NM_CUDA(nmg::launch_fe32_passes(v, b, ctl, s, h->device, h->blocks, chunk, h->ev[3],
                                     h->ev[4], h->fe_overlap ? &o : nullptr, stage,
                                     h->l2_window));

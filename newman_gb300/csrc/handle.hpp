@@ -78,8 +78,8 @@ struct nm_handle {
   // loop (1367x769x4 view at 3e-5: 20.4 -> 19.8 ms, a row of 640 samples 0.39 ->
   // 0.38), else 32
   int fp64_chunk(bool double_loop) const { return chunk > 0 ? chunk : double_loop ? 64 : 32; }
-  // renorm 0: 64 steps a chunk, 32 on floatexp views (measured: 1920x1080x16 at
-  // width 1e-12 190 -> 185 ms with 64; 3840x2160 at width 1e-300 31 -> 33 ms)
+  // renorm 0: 64 steps a chunk (with 32, 64 and 128: 1920x1080x16 at width 1e-12 89.4,
+  // 85.7, 84.7 ms; 3840x2160 at 1e-300 66.0, 63.0, 62.4; 2x2 samples at 1e-412 1,086 each)
   int tile_w = 16, tile_h = 16, chunk = 0, blocks = 0, threads = 0, renorm = 0;
   bool keep_smooth64 = false;
   cudaStream_t stream = nullptr;
@@ -127,7 +127,7 @@ struct nm_handle {
   int reference_mode = nmg::REFERENCE_PROBES;
   // FE32 iteration pass: orbit entries staged in shared memory by the TMA unit
   // (orbit_stage.cuh), and a persisting L2 access-policy window on the orbit
-  int z_stage = -1;  // -1: kAutoOrbitStage on floatexp views, else none
+  int z_stage = -1;  // -1: none
   bool l2_window = false;
   // renders stop every sample at min(N, iter_cap) iterations (0: N); for
   // previews that estimate where the work lies

@@ -204,18 +204,26 @@ __global__ void __launch_bounds__(kPersistentThreads) fe_iter_kernel(DeviceView 
   fe_iter_warp<false, kRawT>(v, b, ctl, chunk);
 }
 
-// The iteration pass with the FP64 rework overlapped: the last two warps of
-// every block render uncertified samples in FP64 (the FP64 pipe is idle under
+// The iteration pass with the FP64 rework overlapped: the last two or three warps
+// of every block render uncertified samples in FP64 (the FP64 pipe is idle under
 // the FP32 iteration) from the start and drain the list to its end; the other
 // warps iterate in FP32 and leave when the FP32 work list is exhausted (the
 // FP64 code under this kernel's 64-register cap spills; a warp joining it
 // made a 3840x2160 (2x2) view of width 1e-413 5 % slower and helped nowhere).
 // Capped at 64 registers so that 4 blocks fit on an SM (3 blocks at 80: the
-// 1920x1080x16 view of width 1e-12 86 ms either way, the 3840x2160 view of width
-// 1e-300 66 against 69 ms).  Two FP64 warps a block; three or four only spread
-// the same FP64 work over more, emptier warps (1e-12 view 86, 89, 100 ms; 1e-300
-// view 66, 66, 73 ms), and with the rework after the pass these take 107 and 88 ms.
-constexpr int kFp64Warps = 2;
+// 1920x1080x16 view of width 1e-12 86 ms either way).  Two FP64 warps a block there:
+// three or four only spread the same FP64 work over more, emptier warps (85, 90, 98
+// ms; with the rework after the pass 112).  Floatexp views and those of many
+// iterations rework more samples, for longer, and take three
+// (2 -> 3 warps: 3840x2160 at 1e-40, N 1e6 114 -> 97 ms, at 1e-120 105 -> 90, at 1e-300
+// 64 -> 63, at 1e-330 184 -> 162, 2x2 samples at 1e-412 1,258 -> 1,086; at 1e-500, where
+// the FP32 side is the longer one, 233 -> 241); four: 69, 163, 1,183, 270 on the
+// last four.  What decides is the share of reworked samples, known only afterwards:
+// from 4 % on three are faster (2x2 at 1e-20, N 50,000 182 -> 157), near 2 % two
+// (1e-60 30.5 -> 28.4 ms with N 100,000 or more).  A sixth FP32 warp that changed
+// sides on a backlog of 32 entries a block came within 2 % of the better of the two
+// on the deep views and gave 88 ms on the 1e-12 one.
+int fp64_warps_for(const DeviceView& v) { return (v.sa_fe || v.N > 200000) ? 3 : 2; }
 
 // The FP64 side, out of line: its register pressure (the FP64 series front)
 // then stays out of the FP32 iteration's allocation.
@@ -230,7 +238,8 @@ __device__ __noinline__ void overlap_fp64_side(const DeviceView& v, const Overla
 // kStaged: the launch stages the orbit's first v.z_stage entries in its
 // dynamic shared memory (orbit_stage.cuh) and both sides read them there.
 // kRawT: the FP32 step's t = 2Z + delta unnormalised (fe_core.cuh, kFeUTRaw).
-template <bool kStaged, bool kRawT>
+// kFp64Warps: the warps of a block on the FP64 side.
+template <bool kStaged, bool kRawT, int kFp64Warps>
 __global__ void __launch_bounds__(kPersistentThreads, 4) fe_overlap_kernel(
     DeviceView v, FePassBuffers b, RenderCtl ctl, OverlapCtl o, int chunk) {
   __shared__ SamplePool<typename Fp64AnyJobT<kStaged>::State> pool;
@@ -306,12 +315,16 @@ cudaError_t launch_fe32_passes(const DeviceView& v, const FePassBuffers& b, cons
     DeviceView vs = v;
     vs.z_stage = z_stage < 0 ? 0 : (z_stage > v.zlen ? v.zlen : z_stage);
     const size_t dyn = 32 * (size_t)vs.z_stage;
-    // Views in the FP64 range take the unnormalised t (C2: 182 -> 170 ms); on
-    // floatexp views its larger bound reworks more samples, and their frame
-    // time is set by the reworked tail (1e-300 view: 31.3 -> 32.9 ms).
+    // Views in the FP64 range take the unnormalised t (1920x1080x16 at 1e-12, before
+    // the jumps: 182 -> 170 ms); on floatexp views its larger bound reworks more
+    // samples, and their frame time is set by the reworked tail (3840x2160 at 1e-300:
+    // 67.8 -> 68.1 ms, 2x2 at 1e-412 1,382 -> 1,411).
     const bool raw_t = fe_raw_t(v);
     auto pick = [&](auto staged, auto raw) {
-      return fe_overlap_kernel<decltype(staged)::value, decltype(raw)::value>;
+      constexpr bool kS = decltype(staged)::value, kR = decltype(raw)::value;
+      // (the normalised t is the floatexp views': three)
+      if (kR && fp64_warps_for(v) == 2) return fe_overlap_kernel<kS, kR, kR ? 2 : 3>;
+      return fe_overlap_kernel<kS, kR, 3>;
     };
     using T_ = std::true_type;
     using F_ = std::false_type;
