@@ -148,7 +148,7 @@ NM_HD int fe_chain_at(const DeviceView& v, int j) {
 // The jump (jump.hpp) of a sample at a chain's first index: its next steps at
 // once, where x = delta + Gamma eps lies in the ball of a record.  The bound
 // passes through the jump by the polynomial's derivative at x: e' = |d delta/dx| e
-// + err.  A bound above 2^-24 |x| keeps the sample from jumping: below it
+// + err, the orders of eps by the largest they reach in the ball.  A bound above 2^-24 |x| keeps the sample from jumping: below it
 // every rebase so far was decided alike in both paths (kFeTie).
 NM_HD void fe_chain_jump(const DeviceView& v, FeState& st) {
   const int c = fe_chain_at(v, st.j);
@@ -252,9 +252,9 @@ NM_HD void fe_chain_jump(const DeviceView& v, FeState& st) {
     gi = fmaf(gr, yh, fmaf(gi, xh, c.y));
     gr = t;
   }
-  // FP32 rounding of it (at most 2^-18 of the sum of its terms) and the second
-  // derivative over the ball of radius ex
-  const float amp = up_fma(use->lip2, ex, up_fma(0x1p-17f, use->lip, approx_norm(gr, gi)));
+  // its FP32 rounding and the derivative of the orders of eps (slack), and the
+  // second derivative over the ball of radius ex
+  const float amp = up_fma(use->lip2, ex, up_add(use->slack, approx_norm(gr, gi)));
   const float err = up_fma(amp, ex, use->err);
   const float sc = use->scale;
   st.dr = FF{dr.h * sc, dr.l * sc};

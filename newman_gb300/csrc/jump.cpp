@@ -69,9 +69,8 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
   if (std::ldexp(rho, -sh) == 0.5) sh--;
   const double rr = std::ldexp(rho, -sh);
   const int k0 = std::ilogb(norm(u.re[0][1], u.im[0][1])) + sh;
-  double mag[D + 1] = {}, err = 0.0, lip = 0.0, rk = 1.0;
+  double mag[D + 1] = {}, err = 0.0, lip = 0.0, lip_eps = 0.0, lip2 = 0.0, rk = 1.0;
   JumpRec o{};
-  double lip2 = 0.0;
   for (int k = 1; k <= D; k++) {
     const double re = std::ldexp(u.re[0][k], sh * k - k0);
     const double im = std::ldexp(u.im[0][k], sh * k - k0);
@@ -114,6 +113,9 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
       // rounded: the coefficient, y^k, at most 3 of 2^-24 a Horner step on the
       // partial sums it is part of, and the product and sum with the next order
       err += ((8.0 + 4.0 * (k + 2.0 * b)) * (ff ? 0x1p-43 : 0x1p-24) * m + 0x1p-100) * rk;
+      // d / dx of it, at most, which the device does not evaluate, and half d2 / dx2
+      if (k > 0) lip_eps += k * m * rk / rr;
+      if (k > 1) lip2 += 0.5 * k * (k - 1) * m * rk / (rr * rr);
       rk *= rr;
     }
   }
@@ -141,7 +143,9 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
   o.scale = (float)pow2(o.s);
   o.rho2 = (float)(rr * rr * (1.0 - 0x1p-20));
   o.err = std::nextafter((float)err, INFINITY);
-  o.lip = (float)(1.01 * lip);
+  // the device's FP32 derivative of order 0 (of its terms' sum, at most 2^-18 in
+  // the Horner steps and 2^-21 in the norm) and the orders of eps
+  o.slack = (float)(1.01 * (0x1p-17 * lip + lip_eps));
   o.lip2 = (float)(2.0 * lip2);
   r = o;
   return true;

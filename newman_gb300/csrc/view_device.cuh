@@ -87,7 +87,9 @@ struct Flt2 {
 };
 struct alignas(16) JumpRec {
   int32_t fire, n, p, s;
-  float rho2, err, lip, lip2;  // bounds of |d delta_n / dx| and of half its second
+  float rho2, err;
+  float slack, lip2;   // |d delta_n / dx| is at most the device's value of order 0's plus
+                       // slack; half the second derivative at most lip2 (chain jumps)
   float unit, scale;   // 2^-p, 2^s (chain jumps)
   int32_t pad_[2];
   Flt4 gamma;          // Gamma (chain jumps)

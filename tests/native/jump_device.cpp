@@ -1,0 +1,142 @@
+// The FP32 path's jumps as the device makes them (newman_gb300/csrc/fe_jump.cuh,
+// its host build) against the records' polynomials in long double.
+//
+//   jump_device what re im step nr nc N probes|center samples seed
+//
+// what = slope: the factor by which a chain jump multiplies a start's bound is at
+// least the derivative of the whole polynomial, orders of eps included, at the
+// start: samples stand at a chain's first index with delta on the edge of a
+// record's ball and eps a corner of the grid, and jump with two bounds.
+//
+// Prints "jumps violations worst", worst the largest ratio.
+#include <cmath>
+#include <complex>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <random>
+#include <string>
+
+#include "../../newman_gb300/csrc/fe_jump.cuh"
+#include "../../newman_gb300/csrc/jump.hpp"
+
+using namespace nmg;
+typedef long double LD;
+typedef std::complex<LD> CL;
+
+static JumpTables tables;
+static std::vector<JumpRec> records;
+static std::vector<RFE> er, ei;
+static DeviceView view;
+
+static CL eps_at(size_t c, size_t r) { return CL(ldexpl(er[c].m, er[c].e), ldexpl(ei[r].m, ei[r].e)); }
+
+static FF ff(LD x) {
+  const float h = (float)x;
+  return FF{h, (float)(x - (LD)h)};
+}
+
+// A sample at the first index of `chain` with delta d, eps and bound e.
+static FeState state(int chain, CL d, CL eps, float e) {
+  FeState st{};
+  st.dr = ff(d.real());
+  st.di = ff(d.imag());
+  st.er = ff(eps.real());
+  st.ei = ff(eps.imag());
+  st.err = e;
+  st.j = view.jump_from[chain];
+  st.i = st.j;
+  st.certified = 1;
+  return st;
+}
+
+// The derivative at x = y 2^p of the record's polynomial, all orders of eps.
+static CL slope(const JumpRec& r, CL y, CL eps) {
+  CL g = 0;
+  for (int k = kJumpDegree; k >= 1; k--) {
+    const CL c = k <= kJumpExact ? CL((LD)r.b[k - 1].x + r.b[k - 1].y, (LD)r.b[k - 1].z + r.b[k - 1].w)
+                                 : CL(r.c[k - kJumpExact - 1].x, r.c[k - kJumpExact - 1].y);
+    g = g * y + (LD)k * c;
+  }
+  const Flt2* tab[4] = {r.q1, r.q2, r.q3, r.q4};
+  const int len[4] = {kJumpEps1, kJumpEps2, kJumpEps3, kJumpEps4};
+  CL e = 1;
+  for (int b = 0; b < 4; b++) {
+    e *= 0x1p32L * eps;
+    CL t = 0;
+    for (int k = len[b] - 1; k >= 1; k--) {
+      CL c(tab[b][k].x, tab[b][k].y);
+      if (b == 0 && k < kEpsExact) c += CL(r.q1l[k].x, r.q1l[k].y);
+      t = t * y + (LD)k * c;
+    }
+    g += t * e;
+  }
+  return g;
+}
+
+// The record of `chain` that a sample jumped by, from its new index.
+static const JumpRec* taken(int chain, const FeState& a, const FeState& b) {
+  for (int i = 0; i < kChainClasses; i++) {
+    const JumpRec& r = tables.chain[(size_t)chain * kChainClasses + i];
+    if (r.rho2 > 0 && r.n - r.fire == b.j - a.j && (float)r.scale != 0.0f) return &r;
+  }
+  return nullptr;
+}
+
+static int check_slope(int samples, std::mt19937_64& g) {
+  std::uniform_real_distribution<double> U(0.0, 1.0);
+  long jumps = 0, bad = 0;
+  LD worst = 0;
+  for (int s = 0; s < samples; s++) {
+    const int chain = (int)(g() % kChains), i = (int)(g() % kChainClasses);
+    const JumpRec& r = tables.chain[(size_t)chain * kChainClasses + i];
+    if (tables.start_index[chain] < 0 || !(r.rho2 > 0)) continue;
+    const CL eps = eps_at(g() % 2 ? 0 : er.size() - 1, g() % 2 ? 0 : ei.size() - 1);
+    // x on the ball's edge, delta = x - Gamma eps
+    const LD a = ldexpl(sqrtl(r.rho2) * (0.9L + 0.09L * U(g)), r.p), ph = 6.2831853L * U(g);
+    const CL gamma((LD)r.gamma.x + r.gamma.y, (LD)r.gamma.z + r.gamma.w);
+    const CL x = CL(a * cosl(ph), a * sinl(ph)), d = x - gamma * eps;
+    const float e = (float)(0x1p-27L * a);
+    FeState st1 = state(chain, d, eps, e), st2 = state(chain, d, eps, 4.0f * e), st0 = st1;
+    fe_chain_jump(view, st1);
+    fe_chain_jump(view, st2);
+    const JumpRec* t = taken(chain, st0, st1);
+    if (st1.j == st0.j || st2.j != st1.j || t != &r) continue;  // by another class's record
+    jumps++;
+    const LD got = ((LD)st2.err - st1.err) / (3 * (LD)e) / r.scale * ldexpl(1, r.p);
+    const LD want = std::abs(slope(r, CL(ldexpl(x.real(), -r.p), ldexpl(x.imag(), -r.p)), eps));
+    // (the bounds' own rounding: 2^-23 of themselves)
+    worst = std::max(worst, want / got);
+    if (want > got * (1 + 0x1p-20L)) bad++;
+  }
+  std::printf("%ld %ld %.7f\n", jumps, bad, (double)worst);
+  return bad ? 1 : 0;
+}
+
+int main(int argc, char** argv) {
+  if (argc != 11) return 2;
+  const char* what = argv[1];
+  MPView v(std::atoi(argv[5]), std::atoi(argv[6]));
+  if (v.set_view(argv[2], argv[3], argv[4], argv[4], std::atoi(argv[7]), 1e-10, 0)) return 3;
+  OrbitData od;
+  const bool center = !std::strcmp(argv[8], "center");
+  if (v.precompute(4, od, center ? REFERENCE_CENTER : REFERENCE_PROBES, false, nullptr, nullptr))
+    return 4;
+  v.eps_tables_fe(er, ei);
+  LD mx = 0, my = 0;
+  for (const RFE& x : er) mx = std::max(mx, fabsl(ldexpl(x.m, x.e)));
+  for (const RFE& y : ei) my = std::max(my, fabsl(ldexpl(y.m, y.e)));
+  const LD m = sqrtl(mx * mx + my * my);
+  build_jumps(od, (double)ldexpl(m, -ilogbl(m)) * (1.0 + 0x1p-40), ilogbl(m), 4, tables);
+  records = tables.start;
+  records.insert(records.end(), tables.chain.begin(), tables.chain.end());
+  view.N = 1 << 30;
+  view.jump = records.data();
+  view.jump_x2 = 0x1p-16f;
+  for (int k = 0; k < kChains; k++)
+    view.jump_from[k] = tables.start_index[k] < 0 ? -1 : tables.start_index[k] + 1;
+  std::mt19937_64 g(std::strtoull(argv[10], nullptr, 10));
+  const int samples = std::atoi(argv[9]);
+  if (!std::strcmp(what, "slope")) return check_slope(samples, g);
+  return 2;
+}

@@ -1,0 +1,43 @@
+"""The FP32 path's jumps as the device makes them (newman_gb300/csrc/fe_jump.cuh in
+its host build, tests/native/jump_device.cpp) against the records' polynomials in
+long double.  CPU only."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from test_jumps import CSRC, CUDA_INC, HERE, ROOT, SEAHORSE, center
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    if not shutil.which("g++"):
+        pytest.skip("no g++")
+    exe = str(tmp_path_factory.mktemp("jump_device") / "jump_device")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-pthread", "-I", CSRC,
+                    "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
+                    os.path.join(HERE, "native", "jump_device.cpp"),
+                    os.path.join(CSRC, "jump.cpp"), os.path.join(CSRC, "mpview.cpp"),
+                    "-o", exe, "-l:libgmp.so.10"], check=True)
+
+    def go(what, where, step, nr, nc, N, mode, samples=20000, seed=5):
+        re, im = where if isinstance(where, tuple) else center(where)
+        out = subprocess.run([exe, what, re, im, step, str(nr), str(nc), str(N), mode,
+                              str(samples), str(seed)], capture_output=True, text=True)
+        assert out.returncode in (0, 1) and out.stdout, out.stderr
+        return out.stdout.split()
+    return go
+
+
+# The whole grid of a 1920x1080x16 view (the largest eps beside the balls), both
+# references; eps small beside most balls; eps below the orders kept.
+@pytest.mark.parametrize("where,step,nr,nc,N,mode", [
+    (SEAHORSE, "1.302083e-16", 4320, 7680, 50000, "probes"),
+    (SEAHORSE, "1.302083e-16", 4320, 7680, 50000, "center"),
+    (18, "1e-18", 541, 961, 50000, "center"),
+    (40, "1e-43", 61, 83, 60000, "center"),
+])
+def test_bound_grows_by_the_whole_derivative(run, where, step, nr, nc, N, mode):
+    jumps, bad, worst = run("slope", where, step, nr, nc, N, mode)
+    assert bad == "0" and int(jumps) > 3000, (jumps, bad, worst)
