@@ -107,8 +107,8 @@ NM_HD void jump_poly(const JumpRec& rec, FF xr, FF xi, FF& dr, FF& di) {
 // The jump (jump.hpp) of a sample that stops the series at `fire`: its delta at
 // the jump's index `found`, within `dbound`; false when it has none.
 // Bit-for-bit the same start in every kernel.
-NM_HD bool fe_jump(const DeviceView& v, int fire, const FFE& er,
-                                        const FFE& ei, CFF& d, float& dbound, int& found) {
+NM_HD bool fe_jump(const DeviceView& v, int fire, const FFE& er, const FFE& ei, CFF& d,
+                   float& dbound, int& found) {
   if (!v.jump) return false;
   const JumpRec* rec = v.jump;
   int c = 0;
@@ -120,8 +120,10 @@ NM_HD bool fe_jump(const DeviceView& v, int fire, const FFE& er,
   // the smallest radius that holds the sample
   const JumpRec* use = nullptr;
   FF xr{0.0f, 0.0f}, xi{0.0f, 0.0f};
+  // (a component that is 0, on the row or column of the reference, has no exponent)
+  const int e = er.h == 0.0f ? ei.e : ei.h == 0.0f ? er.e : er.e > ei.e ? er.e : ei.e;
   for (int k = kJumpSubs - 1; k >= 0 && !use; k--) {
-    if (!(rec[k].rho2 > 0.0f) || (er.e > ei.e ? er.e : ei.e) - rec[k].p > 20) continue;
+    if (!(rec[k].rho2 > 0.0f) || e - rec[k].p > 20) continue;
     xr = ffe_scaled(er.h, er.l, er.e - rec[k].p);
     xi = ffe_scaled(ei.h, ei.l, ei.e - rec[k].p);
     if (fmaf(xr.h, xr.h, xi.h * xi.h) <= rec[k].rho2) use = rec + k;

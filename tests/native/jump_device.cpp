@@ -7,6 +7,8 @@
 // least the derivative of the whole polynomial, orders of eps included, at the
 // start: samples stand at a chain's first index with delta on the edge of a
 // record's ball and eps a corner of the grid, and jump with two bounds.
+// what = start: a sample whose eps lies in a start record's ball, on one of the
+// axes or off them, jumps, to within the bound of the polynomial.
 //
 // Prints "jumps violations worst", worst the largest ratio.
 #include <cmath>
@@ -113,6 +115,56 @@ static int check_slope(int samples, std::mt19937_64& g) {
   return bad ? 1 : 0;
 }
 
+static FFE ffe(LD x) {
+  if (x == 0) return FFE{0.0f, 0.0f, 0, 0};
+  const int k = ilogbl(x);
+  const FF m = ff(ldexpl(x, -k));
+  return FFE{m.h, m.l, k, 0};
+}
+
+static int check_start(int samples, std::mt19937_64& g) {
+  std::uniform_real_distribution<double> U(0.0, 1.0);
+  long jumps = 0, bad = 0;
+  LD worst = 0;
+  for (int s = 0; s < samples; s++) {
+    const JumpRec& r = tables.start[g() % tables.start.size()];
+    if (!(r.rho2 > 0)) continue;
+    const LD a = ldexpl(sqrtl(r.rho2) * (0.5L + 0.49L * U(g)), r.p), ph = 6.2831853L * U(g);
+    const int axis = (int)(g() % 3);
+    const FFE fr = ffe(axis == 0 ? 0 : axis == 1 ? a : a * cosl(ph));
+    const FFE fi = ffe(axis == 0 ? -a : axis == 1 ? 0 : a * sinl(ph));
+    CFF d;
+    float bound = 0.0f;
+    int found = -1;
+    if (!fe_jump(view, r.fire, fr, fi, d, bound, found)) {
+      bad++;
+      continue;
+    }
+    jumps++;
+    // the record it took: the smallest radius that holds it
+    const JumpRec* use = nullptr;
+    for (const JumpRec& q : tables.start)
+      if (q.fire == r.fire && q.rho2 > 0 && q.n == found && q.err == bound && q.s == d.e) use = &q;
+    if (!use) {
+      bad++;
+      continue;
+    }
+    const CL y(ldexpl((LD)fr.h + fr.l, fr.e - use->p), ldexpl((LD)fi.h + fi.l, fi.e - use->p));
+    CL p = 0;
+    for (int k = kJumpDegree; k >= 1; k--) {
+      const CL c = k <= kJumpExact
+                       ? CL((LD)use->b[k - 1].x + use->b[k - 1].y, (LD)use->b[k - 1].z + use->b[k - 1].w)
+                       : CL(use->c[k - kJumpExact - 1].x, use->c[k - kJumpExact - 1].y);
+      p = (p + c) * y;
+    }
+    const LD e = std::abs(p - CL((LD)d.re.h + d.re.l, (LD)d.im.h + d.im.l)) / bound;
+    worst = std::max(worst, e);
+    if (!(e <= 1)) bad++;
+  }
+  std::printf("%ld %ld %.7f\n", jumps, bad, (double)worst);
+  return bad ? 1 : 0;
+}
+
 int main(int argc, char** argv) {
   if (argc != 11) return 2;
   const char* what = argv[1];
@@ -138,5 +190,6 @@ int main(int argc, char** argv) {
   std::mt19937_64 g(std::strtoull(argv[10], nullptr, 10));
   const int samples = std::atoi(argv[9]);
   if (!std::strcmp(what, "slope")) return check_slope(samples, g);
+  if (!std::strcmp(what, "start")) return check_start(samples, g);
   return 2;
 }

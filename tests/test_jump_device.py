@@ -41,3 +41,14 @@ def run(tmp_path_factory):
 def test_bound_grows_by_the_whole_derivative(run, where, step, nr, nc, N, mode):
     jumps, bad, worst = run("slope", where, step, nr, nc, N, mode)
     assert bad == "0" and int(jumps) > 3000, (jumps, bad, worst)
+
+
+# One component of eps exactly 0: the row and the column of a view-center reference.
+@pytest.mark.parametrize("where,step,nr,nc,N,mode", [
+    (SEAHORSE, "1e-17", 37, 65, 50000, "center"),
+    (18, "1e-18", 541, 961, 50000, "center"),
+    (160, "1e-163", 48, 64, 130000, "center"),
+])
+def test_start_jumps_on_the_axes(run, where, step, nr, nc, N, mode):
+    jumps, bad, worst = run("start", where, step, nr, nc, N, mode)
+    assert bad == "0" and int(jumps) > 1000, (jumps, bad, worst)
