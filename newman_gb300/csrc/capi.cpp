@@ -279,26 +279,14 @@ void build_front32_tables(nm_handle* h, bool series = true) {
 
 // The FP32 path's jumps (jump.hpp), for |eps| up to the farthest sample's.
 void build_jump_tables(nm_handle* h, int threads) {
-  double mx = 0.0, my = 0.0;
-  int e = 0;
-  if (h->od.sa_fp64_ok) {
-    for (double x : h->eps_re) mx = std::max(mx, std::fabs(x));
-    for (double y : h->eps_im) my = std::max(my, std::fabs(y));
-  } else {
-    // every component at the largest exponent
-    e = -(1 << 30);
-    for (const nmg::RFE& x : h->eps_re_fe)
-      if (x.m != 0.0) e = std::max(e, x.e + std::ilogb(x.m));
-    for (const nmg::RFE& y : h->eps_im_fe)
-      if (y.m != 0.0) e = std::max(e, y.e + std::ilogb(y.m));
-    for (const nmg::RFE& x : h->eps_re_fe) mx = std::max(mx, std::fabs(std::scalbn(x.m, x.e - e)));
-    for (const nmg::RFE& y : h->eps_im_fe) my = std::max(my, std::fabs(std::scalbn(y.m, y.e - e)));
-  }
-  const double m = std::sqrt(mx * mx + my * my) * (1.0 + 0x1p-40);
+  const nmg::EpsRange range = h->od.sa_fp64_ok ? nmg::eps_range(h->eps_re, h->eps_im)
+                                               : nmg::eps_range(h->eps_re_fe, h->eps_im_fe);
   nmg::JumpTables t;
-  nmg::build_jumps(h->od, m, e, threads, t);
+  nmg::build_jumps(h->od, range.norm(), range.e, threads, t);
   h->jump = std::move(t.start);
   h->jump.insert(h->jump.end(), t.chain.begin(), t.chain.end());
+  h->jump_er = range.re_limit();
+  h->jump_ei = range.im_limit();
   h->jump_x2 = 0.0f;
   for (int k = 0; k < nmg::kChains; k++) {
     // X[s] is z[s + 1]
@@ -328,6 +316,8 @@ void set_fe_tables(const nm_handle* h, nmg::DeviceView& v) {
     v.jump = t->jump.empty() ? nullptr : t->d_jump.p;
     std::copy(t->jump_from, t->jump_from + nmg::kChains, v.jump_from);
     v.jump_x2 = t->jump_x2;
+    v.jump_er = t->jump_er;
+    v.jump_ei = t->jump_ei;
   }
   v.sa_fe = h->od.sa_fp64_ok ? 0 : 1;
   if (!v.sa_fe) return;
@@ -479,6 +469,8 @@ nm_handle* nm_copy(const nm_handle* src) {
   h->jump = src->jump;
   std::copy(src->jump_from, src->jump_from + nmg::kChains, h->jump_from);
   h->jump_x2 = src->jump_x2;
+  h->jump_er = src->jump_er;
+  h->jump_ei = src->jump_ei;
   h->reference_mode = src->reference_mode;
   h->fe_single_pass = src->fe_single_pass;
   h->fe_overlap = src->fe_overlap;

@@ -156,7 +156,7 @@ NM_HD void fe_chain_jump(const DeviceView& v, FeState& st) {
   const int c = fe_chain_at(v, st.j);
   if (c < 0) return;
   const float x2 = fmaf(st.dr.h, st.dr.h, st.di.h * st.di.h);
-  if (!(x2 < v.jump_x2)) return;
+  if (!(x2 < v.jump_x2) || fabsf(st.er.h) > v.jump_er || fabsf(st.ei.h) > v.jump_ei) return;
   // class i: |x|^2 < 2^-(kChainTop + 2 i), i from the exponent of |delta|^2
   int i = (126 - kChainTop - (float_bits(x2) >> 23)) >> 1;
   const JumpRec* base = v.jump + kJumpClasses * kJumpSubs + c * kChainClasses;

@@ -119,7 +119,7 @@ struct nm_handle {
   std::vector<nmg::TFE> sa_min32;
   std::vector<nmg::JumpRec> jump;
   int32_t jump_from[nmg::kChains] = {};
-  float jump_x2 = 0.0f;
+  float jump_x2 = 0.0f, jump_er = 0.0f, jump_ei = 0.0f;
   DevBuf<nmg::FFE> d_eps32_re, d_eps32_im;
   DevBuf<nmg::CFFE> d_a32, d_b32, d_c32;
   DevBuf<nmg::TFE> d_sa_min32;

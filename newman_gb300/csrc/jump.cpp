@@ -637,6 +637,24 @@ void build_chain(const OrbitData& od, int s, double eps, JumpRec* out, int* stop
 
 }  // namespace
 
+EpsRange eps_range(const std::vector<double>& re, const std::vector<double>& im) {
+  EpsRange r{0.0, 0.0, 0};
+  for (double x : re) r.re = std::max(r.re, std::fabs(x));
+  for (double y : im) r.im = std::max(r.im, std::fabs(y));
+  return r;
+}
+
+EpsRange eps_range(const std::vector<RFE>& re, const std::vector<RFE>& im) {
+  // every component at the largest exponent
+  EpsRange r{0.0, 0.0, -(1 << 30)};
+  for (const auto* v : {&re, &im})
+    for (const RFE& x : *v)
+      if (x.m != 0.0) r.e = std::max(r.e, x.e + std::ilogb(x.m));
+  for (const RFE& x : re) r.re = std::max(r.re, std::fabs(std::scalbn(x.m, x.e - r.e)));
+  for (const RFE& y : im) r.im = std::max(r.im, std::fabs(std::scalbn(y.m, y.e - r.e)));
+  return r;
+}
+
 void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t) {
   JumpRec none{};
   none.rho2 = -1.0f;

@@ -34,6 +34,7 @@
 // step, the same for both paths while they are at the same element.
 #pragma once
 
+#include <cmath>
 #include <vector>
 
 #include "mpview.hpp"
@@ -47,6 +48,18 @@ struct JumpTables {
                                  // 2^-(kChainTop + 2 i)); unused: rho2 -1
   std::vector<int> start_index;  // kChains: X index each starts at; -1: none
 };
+
+// The largest |component|s of a grid's eps: re 2^e and im 2^e.
+struct EpsRange {
+  double re, im;
+  int e;
+  double norm() const { return std::sqrt(re * re + im * im) * (1.0 + 0x1p-40); }
+  // as floats, not below them
+  float re_limit() const { return std::nextafter((float)std::scalbn(re, e), INFINITY); }
+  float im_limit() const { return std::nextafter((float)std::scalbn(im, e), INFINITY); }
+};
+EpsRange eps_range(const std::vector<double>& re, const std::vector<double>& im);
+EpsRange eps_range(const std::vector<RFE>& re, const std::vector<RFE>& im);
 
 // The tables of a precomputed deep view whose samples have |eps| <= m 2^e.
 void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t);

@@ -159,6 +159,8 @@ struct DeviceView {
                            // or null
   int32_t jump_from[kChains];  // orbit indexes j (of z) of the chains' starts; -1: none
   float jump_x2;           // starts with |delta|^2 below it may jump (0: none)
+  float jump_er, jump_ei;  // chain jumps hold for |eps| components up to these (a
+                           // preview's rows can lie outside its source's grid)
 
   // the reference-exact path: values in the view's arbitrary precision as
   // records of mp_limbs limbs (mpf_fixed.cuh; word 0: exponent << 32 | sign)

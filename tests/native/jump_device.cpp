@@ -7,6 +7,10 @@
 // least the derivative of the whole polynomial, orders of eps included, at the
 // start: samples stand at a chain's first index with delta on the edge of a
 // record's ball and eps a corner of the grid, and jump with two bounds.
+// what = range: eps at a corner of the grid jumps, eps beyond it in one component
+// does not (a preview's last row can lie outside the grid of the view whose tables it
+// shares).  "violations": jumps beyond; "worst": the part of those inside that jump.
+//
 // what = start: a sample whose eps lies in a start record's ball, on one of the
 // axes or off them, jumps, to within the bound of the polynomial.
 //
@@ -30,6 +34,7 @@ static JumpTables tables;
 static std::vector<JumpRec> records;
 static std::vector<RFE> er, ei;
 static DeviceView view;
+static EpsRange range;
 
 static CL eps_at(size_t c, size_t r) { return CL(ldexpl(er[c].m, er[c].e), ldexpl(ei[r].m, ei[r].e)); }
 
@@ -115,6 +120,38 @@ static int check_slope(int samples, std::mt19937_64& g) {
   return bad ? 1 : 0;
 }
 
+static int check_range(int samples, std::mt19937_64& g) {
+  std::uniform_real_distribution<double> U(0.0, 1.0);
+  long inside = 0, jumped = 0, bad = 0;
+  for (int s = 0; s < samples; s++) {
+    const int chain = (int)(g() % kChains), i = (int)(g() % kChainClasses);
+    const JumpRec& r = tables.chain[(size_t)chain * kChainClasses + i];
+    if (tables.start_index[chain] < 0 || !(r.rho2 > 0)) continue;
+    CL eps = eps_at(g() % 2 ? 0 : er.size() - 1, g() % 2 ? 0 : ei.size() - 1);
+    // the corners that are the farthest in both components
+    if (fabsl(eps.real()) != ldexpl(range.re, range.e) || fabsl(eps.imag()) != ldexpl(range.im, range.e))
+      continue;
+    const LD a = ldexpl(0.7L * sqrtl(r.rho2), r.p), ph = 6.2831853L * U(g);
+    const CL gamma((LD)r.gamma.x + r.gamma.y, (LD)r.gamma.z + r.gamma.w);
+    const LD f = 1.0L + std::exp2(-20.0 + 20.0 * U(g));
+    for (int beyond = 0; beyond < 3; beyond++) {
+      const CL e(beyond == 1 ? f * eps.real() : eps.real(), beyond == 2 ? f * eps.imag() : eps.imag());
+      const CL d = CL(a * cosl(ph), a * sinl(ph)) - gamma * e;
+      FeState st = state(chain, d, e, (float)(0x1p-27L * a));
+      const int j = st.j;
+      fe_chain_jump(view, st);
+      if (beyond == 0) {
+        inside++;
+        jumped += st.j != j;
+      } else {
+        bad += st.j != j;
+      }
+    }
+  }
+  std::printf("%ld %ld %.7f\n", jumped, bad, (double)jumped / std::max(1L, inside));
+  return bad ? 1 : 0;
+}
+
 static FFE ffe(LD x) {
   if (x == 0) return FFE{0.0f, 0.0f, 0, 0};
   const int k = ilogbl(x);
@@ -175,21 +212,21 @@ int main(int argc, char** argv) {
   if (v.precompute(4, od, center ? REFERENCE_CENTER : REFERENCE_PROBES, false, nullptr, nullptr))
     return 4;
   v.eps_tables_fe(er, ei);
-  LD mx = 0, my = 0;
-  for (const RFE& x : er) mx = std::max(mx, fabsl(ldexpl(x.m, x.e)));
-  for (const RFE& y : ei) my = std::max(my, fabsl(ldexpl(y.m, y.e)));
-  const LD m = sqrtl(mx * mx + my * my);
-  build_jumps(od, (double)ldexpl(m, -ilogbl(m)) * (1.0 + 0x1p-40), ilogbl(m), 4, tables);
+  range = eps_range(er, ei);
+  build_jumps(od, range.norm(), range.e, 4, tables);
   records = tables.start;
   records.insert(records.end(), tables.chain.begin(), tables.chain.end());
   view.N = 1 << 30;
   view.jump = records.data();
   view.jump_x2 = 0x1p-16f;
+  view.jump_er = range.re_limit();
+  view.jump_ei = range.im_limit();
   for (int k = 0; k < kChains; k++)
     view.jump_from[k] = tables.start_index[k] < 0 ? -1 : tables.start_index[k] + 1;
   std::mt19937_64 g(std::strtoull(argv[10], nullptr, 10));
   const int samples = std::atoi(argv[9]);
   if (!std::strcmp(what, "slope")) return check_slope(samples, g);
+  if (!std::strcmp(what, "range")) return check_range(samples, g);
   if (!std::strcmp(what, "start")) return check_start(samples, g);
   return 2;
 }

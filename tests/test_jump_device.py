@@ -52,3 +52,13 @@ def test_bound_grows_by_the_whole_derivative(run, where, step, nr, nc, N, mode):
 def test_start_jumps_on_the_axes(run, where, step, nr, nc, N, mode):
     jumps, bad, worst = run("start", where, step, nr, nc, N, mode)
     assert bad == "0" and int(jumps) > 1000, (jumps, bad, worst)
+
+
+# eps beyond the grid that the tables were built for, by 2^-20 to 2 times.
+@pytest.mark.parametrize("where,step,nr,nc,N,mode", [
+    (SEAHORSE, "1e-17", 37, 65, 50000, "center"),
+    (18, "1e-18", 541, 961, 50000, "center"),
+])
+def test_no_chain_jump_beyond_the_grid(run, where, step, nr, nc, N, mode):
+    inside, beyond, part = run("range", where, step, nr, nc, N, mode)
+    assert beyond == "0" and int(inside) > 500 and float(part) > 0.5, (inside, beyond, part)
