@@ -822,7 +822,7 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
   if (blocks > need_blocks) blocks = (int)need_blocks;
   if (blocks < 1) blocks = 1;
   int chunk = h->fp64_chunk(kind == nmg::KERNEL_HW || kind == nmg::KERNEL_HW_MP);
-  if (kind == nmg::KERNEL_FE32)  // the FE32 kernel renormalises per chunk
+  if (kind == nmg::KERNEL_FE32)  // steps a round of a warp, and between renormalisations
     chunk = h->renorm > 0 ? h->renorm : 64;
   NM_CUDA(cudaEventRecord(h->ev[0], s));
   h->timed_iter = false;

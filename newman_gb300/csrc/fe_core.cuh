@@ -192,7 +192,7 @@ __device__ __forceinline__ void fe_start(const DeviceView& v, const SeriesFront&
   st.certified = 1;
   st.frame = 0;
   st.e64 = 0.0f;
-  st.pad_ = 0;
+  st.since = 0;
 }
 
 // ---- the series front on the FP32 pipe ---------------------------------------
@@ -328,7 +328,7 @@ __device__ __forceinline__ int fe_front32(const DeviceView& v, int r, int c, FeS
   st.certified = 1;
   st.frame = 0;
   st.e64 = 0.0f;
-  st.pad_ = 0;
+  st.since = 0;
   return kFront32Ready;
 }
 
@@ -412,10 +412,11 @@ __device__ __forceinline__ void fe_renormalise(FeState& st) {
 // 0 that |Y| < |delta| could hold (left to the FP64 kernel: uncertified).
 template <bool kStaged = false, bool kRawT = false>
 __device__ __forceinline__ bool fe_scaled_steps(const DeviceView& v, FeState& st, int steps,
-                                             FeResult& res, unsigned long long& executed,
+                                             int renorm, FeResult& res,
+                                             unsigned long long& executed,
                                              unsigned long long& rebases) {
   const int zlast = v.zlen - 1;
-  const int stop = min(v.N, st.i + steps);
+  const int stop = min(v.N, st.i + min(steps, renorm - st.since));
   const int start = st.i;
   ZFF z = fe_load_z<kStaged>(v, st.j);
   bool done = false;
@@ -501,7 +502,14 @@ __device__ __forceinline__ bool fe_scaled_steps(const DeviceView& v, FeState& st
     }
   }
   executed += (unsigned long long)(st.i - start);
-  if (!done && st.E != 0) fe_renormalise(st);
+  // counted per sample: how its steps are divided into calls depends on the other
+  // lanes of its warp, and must not change its bits
+  st.since += st.i - start;
+  if (!done && st.E != 0 &&
+      (st.since >= renorm || fmaxf(fabsf(st.dr.h), fabsf(st.di.h)) > 0x1p60f)) {
+    fe_renormalise(st);
+    st.since = 0;
+  }
   if (done) return true;
   if (st.i >= v.N) {
     res.it = v.N;
@@ -701,14 +709,14 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
 
 template <bool kStaged = false, bool kRawT = false>
 __device__ __forceinline__ bool fe_advance(const DeviceView& v, FeState& st, int steps,
-                                           FeResult& res, unsigned long long& executed,
+                                           int renorm, FeResult& res, unsigned long long& executed,
                                            unsigned long long& rebases, FeTrap* trap = nullptr) {
   if (st.E != 0) {
     if (v.double_loop) {  // a start below 2^-60: left to the double loop
       st.certified = 0;
       return true;
     }
-    return fe_scaled_steps<kStaged, kRawT>(v, st, steps, res, executed, rebases);
+    return fe_scaled_steps<kStaged, kRawT>(v, st, steps, renorm, res, executed, rebases);
   }
   if (v.double_loop)
     return fe_unscaled_steps<true, kStaged, kRawT>(v, st, steps, res, executed, rebases, trap);

@@ -66,7 +66,7 @@ struct alignas(16) FeState {
   int32_t certified;
   int32_t frame;  // frame of a batch
   float e64;      // double-loop views: bound on the double loop's own error
-  int32_t pad_;
+  int32_t since;  // steps since the exponent was set (while E != 0)
 };
 
 struct CFF {  // ((re) + i (im)) * 2^e, float-float mantissas

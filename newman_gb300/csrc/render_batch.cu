@@ -137,8 +137,8 @@ __device__ __forceinline__ void batch_iter_warp(const BatchGroup& grp, const FeP
     // delta unnormalised on frames inside the FP64 range
     const bool done = fe_round(v, st, active, chunk, [&](int n) {
       FeTrap* trap = v.trap ? v.trap + (g - grp.offsets[f]) : nullptr;
-      return fe_raw_t(v) ? fe_advance<false, true>(v, st, n, res, executed, rebases, trap)
-                         : fe_advance<false, false>(v, st, n, res, executed, rebases, trap);
+      return fe_raw_t(v) ? fe_advance<false, true>(v, st, n, chunk, res, executed, rebases, trap)
+                         : fe_advance<false, false>(v, st, n, chunk, res, executed, rebases, trap);
     });
     if (done) {
       int r = 0, c = 0;

@@ -55,7 +55,7 @@ struct FeJob {
                                                unsigned long long& rebases) {
     FeResult res;
     if (fe_may_jump(v, st)) fe_chain_jump(v, st);
-    if (!fe_advance<false, kRawT>(v, st, n, res, executed, rebases)) return false;
+    if (!fe_advance<false, kRawT>(v, st, n, n, res, executed, rebases)) return false;
     const float s = fe_smoothing(v, res);
     sm = s;
     out = {res.it, s};
@@ -167,7 +167,7 @@ __device__ __forceinline__ void fe_iter_warp(const DeviceView& v, const FePassBu
     if (!__any_sync(kFull, active)) break;
     FeResult res;
     const bool done = fe_round(v, st, active, chunk, [&](int n) {
-      return fe_advance<kStaged, kRawT>(v, st, n, res, executed, rebases,
+      return fe_advance<kStaged, kRawT>(v, st, n, chunk, res, executed, rebases,
                                         v.trap ? v.trap + sid : nullptr);
     });
     if (done) {
