@@ -90,15 +90,6 @@ constexpr float kFeQuickErr = 0.2f;
 constexpr float kFeQuickErrInner = 200.0f;
 constexpr float kFeInner2 = 262144.0f;
 
-// A rebase test |Y|^2 < |delta|^2 nearer to a tie than this may come out unlike in
-// FP32 and FP64: the sample ends uncertified, so that on the others both paths
-// rebase at the same steps for as long as their bound is small.  (The estimates
-// are within 2^-20; a bound of 2^-23 |delta| on each path moves the squares by
-// 2^-20.)  With a
-// larger bound a sample no longer jumps (fe_chain_jump).
-constexpr float kFeTie = 0x1p-19f;
-constexpr float kFeTied = 0x1p-46f;  // ... while the bound is below 2^-23 |delta|
-
 // Interior orbits on double-loop views.  The reference's double loop F (one
 // step z -> z^2 + c in doubles, mandelbrot.cpp:242-246) rounds by at most
 //   |F(z) - f(z)| <= 2^-53 (3|z|^2 + |F(z)|_1) (1 + 2^-52),   f(z) = z^2 + c,
@@ -628,7 +619,7 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
     }
     const float d2 = fmaf(dr.h, dr.h, di.h * di.h);
     if (r2 < (kDl ? d2 : d2 * (1.0f + kFeTie)) || j == zlast) {
-      if (!kDl && j != zlast && r2 >= d2 * (1.0f - kFeTie) && err * err < kFeTied * d2) {
+      if (!kDl && j != zlast && fe_tied(r2, d2, err)) {
         certified = false;
         done = true;
         i++;

@@ -57,6 +57,19 @@ NM_HD float approx_norm(float x, float y) {
   return approx_sqrt(fmaf(x, x, y * y));
 }
 
+// A rebase test |Y|^2 < |delta|^2 nearer to a tie than this may come out unlike in
+// FP32 and FP64: the sample ends uncertified, so that on the others both paths
+// rebase at the same steps for as long as their bound is small.  (The estimates
+// are within 2^-20; a bound of 2^-23 |delta| on each path moves the squares by
+// 2^-20.)  With a larger bound a sample no longer jumps (fe_chain_jump).
+constexpr float kFeTie = 0x1p-19f;
+// r2 = |Y|^2 below d2 (1 + kFeTie), d2 = |delta|^2: near the tie, with a bound below
+// 2^-23 |delta|.  (Compared as magnitudes: their squares leave the float range from
+// |delta| = 2^-52 down.  approx_sqrt's floor only takes in more.)
+NM_HD bool fe_tied(float r2, float d2, float err) {
+  return r2 >= d2 * (1.0f - kFeTie) && err < 0x1p-23f * approx_sqrt(d2);
+}
+
 struct alignas(16) FeState {
   FF dr, di;      // delta * 2^-E
   FF er, ei;      // eps * 2^-E

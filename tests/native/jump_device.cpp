@@ -13,6 +13,8 @@
 //
 // what = start: a sample whose eps lies in a start record's ball, on one of the
 // axes or off them, jumps, to within the bound of the polynomial.
+// what = tie: a rebase test near its tie counts as tied at every size of delta that
+// the unscaled steps meet, as long as the bound is below 2^-23 |delta|.
 //
 // Prints "jumps violations worst", worst the largest ratio.
 #include <cmath>
@@ -202,9 +204,27 @@ static int check_start(int samples, std::mt19937_64& g) {
   return bad ? 1 : 0;
 }
 
+static int check_tie(int samples, std::mt19937_64& g) {
+  std::uniform_real_distribution<double> U(0.0, 1.0);
+  long bad = 0;
+  for (int s = 0; s < samples; s++) {
+    const double d = std::exp2(-59.0 * U(g)), near = (2.0 * U(g) - 1.0) * 0x1p-20;
+    const float d2 = (float)(d * d), r2 = (float)(d * d * (1.0 + near));
+    const double e = std::exp2(-40.0 * U(g));  // bound / |delta|
+    if (e > 0x1p-24 && e < 0x1p-22) continue;
+    if (fe_tied(r2, d2, (float)(e * d)) != (e < 0x1p-23)) bad++;
+    if (fe_tied((float)(d * d * (1.0 - 0x1p-17)), d2, (float)(e * d))) bad++;
+  }
+  std::printf("%d %ld 0\n", samples, bad);
+  return bad ? 1 : 0;
+}
+
 int main(int argc, char** argv) {
   if (argc != 11) return 2;
   const char* what = argv[1];
+  std::mt19937_64 g(std::strtoull(argv[10], nullptr, 10));
+  const int samples = std::atoi(argv[9]);
+  if (!std::strcmp(what, "tie")) return check_tie(samples, g);
   MPView v(std::atoi(argv[5]), std::atoi(argv[6]));
   if (v.set_view(argv[2], argv[3], argv[4], argv[4], std::atoi(argv[7]), 1e-10, 0)) return 3;
   OrbitData od;
@@ -223,8 +243,6 @@ int main(int argc, char** argv) {
   view.jump_ei = range.im_limit();
   for (int k = 0; k < kChains; k++)
     view.jump_from[k] = tables.start_index[k] < 0 ? -1 : tables.start_index[k] + 1;
-  std::mt19937_64 g(std::strtoull(argv[10], nullptr, 10));
-  const int samples = std::atoi(argv[9]);
   if (!std::strcmp(what, "slope")) return check_slope(samples, g);
   if (!std::strcmp(what, "range")) return check_range(samples, g);
   if (!std::strcmp(what, "start")) return check_start(samples, g);

@@ -62,3 +62,8 @@ def test_start_jumps_on_the_axes(run, where, step, nr, nc, N, mode):
 def test_no_chain_jump_beyond_the_grid(run, where, step, nr, nc, N, mode):
     inside, beyond, part = run("range", where, step, nr, nc, N, mode)
     assert beyond == "0" and int(inside) > 500 and float(part) > 0.5, (inside, beyond, part)
+
+
+def test_ties_of_the_rebase_test_at_every_size(run):
+    samples, bad, _ = run("tie", SEAHORSE, "1e-17", 37, 65, 1000, "center")
+    assert bad == "0", bad
