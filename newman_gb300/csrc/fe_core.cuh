@@ -619,13 +619,18 @@ __device__ __forceinline__ bool fe_unscaled_steps(const DeviceView& v, FeState& 
     }
     const float d2 = fmaf(dr.h, dr.h, di.h * di.h);
     if (r2 < (kDl ? d2 : d2 * (1.0f + kFeTie)) || j == zlast) {
+      bool rebase = r2 < d2 || j == zlast;
       if (!kDl && j != zlast && fe_tied(r2, d2, err)) {
-        certified = false;
-        done = true;
-        i++;
-        break;
+        const int side = fe_tie_side(z.hx, z.hy, dr.h, di.h, d2);
+        if (side < 0) {
+          certified = false;
+          done = true;
+          i++;
+          break;
+        }
+        rebase = side == 1;
       }
-      if (r2 < d2 || j == zlast) {  // rebase to Z[0]: delta = Y in float-float
+      if (rebase) {  // to Z[0]: delta = Y in float-float
         const float yerr_fe = y_err();
         const FF nyr = ff_add(FF{z.hx, z.lx}, dr);
         const FF nyi = ff_add(FF{z.hy, z.ly}, di);

@@ -16,6 +16,9 @@
 // what = tie: a rebase test near its tie counts as tied at every size of delta that
 // the unscaled steps meet, as long as the bound is below 2^-23 |delta|.
 //
+// what = side: near a tie, what fe_tie_side decides is what the FP64 path's sums give
+// for both paths' deltas; "worst": the part decided where |Z| > 2^-26 |delta|.
+//
 // Prints "jumps violations worst", worst the largest ratio.
 #include <cmath>
 #include <complex>
@@ -219,12 +222,48 @@ static int check_tie(int samples, std::mt19937_64& g) {
   return bad ? 1 : 0;
 }
 
+static int check_side(int samples, std::mt19937_64& g) {
+  std::uniform_real_distribution<double> U(-1.0, 1.0);
+  long bad = 0, n = 0, decided = 0;
+  for (int s = 0; s < samples; s++) {
+    // delta of any size, Z from as large down to far below its rounding
+    const double d = std::exp2(29.5 * (U(g) - 1.0)), q = std::exp2(25.0 * (U(g) - 1.0));
+    const double p1 = 3.15 * U(g);
+    double dx = d * std::cos(p1), dy = d * std::sin(p1);
+    // Z at an angle of delta with |Z + delta| near |delta|: cos = -q / 2, moved
+    const double c = -0.5 * q + (g() % 2 ? U(g) : U(g) * std::exp2(-24.0 * std::fabs(U(g))));
+    if (std::fabs(c) > 1.0) continue;
+    const double h = std::sqrt(1.0 - c * c) * (g() % 2 ? 1.0 : -1.0);
+    const double zx = q * (dx * c - dy * h), zy = q * (dy * c + dx * h);
+    const float fx = (float)dx, fy = (float)dy, wx = (float)zx, wy = (float)zy;
+    const float yx = wx + fx, yy = wy + fy;
+    const float r2 = fmaf(yx, yx, yy * yy), d2 = fmaf(fx, fx, fy * fy);
+    if (!(r2 < d2 * (1.0f + kFeTie)) || !fe_tied(r2, d2, 0.0f)) continue;
+    n++;
+    const int side = fe_tie_side(wx, wy, fx, fy, d2);
+    if (q > 0x1p-26) decided += side >= 0;
+    else n--;
+    if (side < 0) continue;
+    // the FP64 path's delta, up to 2^-23 off
+    for (int k = 0; k < 4; k++) {
+      const double t = k ? 0x1p-23 * d : 0.0, p2 = 3.15 * U(g);
+      const double ex = dx + t * std::cos(p2), ey = dy + t * std::sin(p2);
+      const double vx = zx + ex, vy = zy + ey;
+      const bool rebase = vx * vx + vy * vy < ex * ex + ey * ey;
+      if (rebase != (side == 1)) bad++;
+    }
+  }
+  std::printf("%ld %ld %.4f\n", n, bad, (double)decided / std::max(1L, n));
+  return bad ? 1 : 0;
+}
+
 int main(int argc, char** argv) {
   if (argc != 11) return 2;
   const char* what = argv[1];
   std::mt19937_64 g(std::strtoull(argv[10], nullptr, 10));
   const int samples = std::atoi(argv[9]);
   if (!std::strcmp(what, "tie")) return check_tie(samples, g);
+  if (!std::strcmp(what, "side")) return check_side(samples, g);
   MPView v(std::atoi(argv[5]), std::atoi(argv[6]));
   if (v.set_view(argv[2], argv[3], argv[4], argv[4], std::atoi(argv[7]), 1e-10, 0)) return 3;
   OrbitData od;

@@ -67,3 +67,8 @@ def test_no_chain_jump_beyond_the_grid(run, where, step, nr, nc, N, mode):
 def test_ties_of_the_rebase_test_at_every_size(run):
     samples, bad, _ = run("tie", SEAHORSE, "1e-17", 37, 65, 1000, "center")
     assert bad == "0", bad
+
+
+def test_side_of_a_tie_is_the_fp64_path_s(run):
+    ties, bad, decided = run("side", SEAHORSE, "1e-17", 37, 65, 1000, "center", samples=2000000)
+    assert bad == "0" and int(ties) > 10000 and float(decided) > 0.5, (ties, bad, decided)
