@@ -559,7 +559,7 @@ def run_ours(args):
     h2d = 16 * (NC * SC + NR * SC) + 8 * (NC * SC + NR * SC)
     xlen = m.stat(nm.STAT_ORBIT_LENGTH)
     h2d += xlen * 16 * 6 + xlen * 8 + (xlen + 2) * 16
-    h2d += 560 * (12 * 7 + 3 * 36)  # the FE32 path's jump records
+    h2d += 576 * (12 * 7 + 3 * 36)  # the FE32 path's jump records
 
     line = None
     if rank == 0:

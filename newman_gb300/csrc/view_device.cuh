@@ -70,7 +70,11 @@ constexpr int32_t kTfeInf = 0x7fffffff, kTfeZero = -0x7fffffff;
 // e = 2^32 eps, within err 2^s, the distance of the FP64 path's own delta_n
 // included.
 constexpr int kJumpDegree = 16;
-constexpr int kJumpExact = 7;     // terms in float-float; the rest in FP32
+// Terms in float-float; the rest (below 2^-20 of the first) in FP32.  With 7 some
+// records' x^8 and x^9 made a jump less near than the float-float steps it stands for,
+// and the smoothing of a 1920x1080 view at 1e-20 up to 1.2e-4 off the FP64 path's
+// (3.4e-5 with 9); 10 and 12 change nothing.
+constexpr int kJumpExact = 9;
 // Orders of eps (chain jumps), with terms; order 1's constant is 0 but where a
 // record could not be centred on it, and its first kEpsExact terms are in
 // float-float.

@@ -13,6 +13,11 @@
 //
 // what = start: a sample whose eps lies in a start record's ball, on one of the
 // axes or off them, jumps, to within the bound of the polynomial.
+// what = precision: against the exact iteration, jumps are off by no more than the
+// float-float steps they stand for, root mean square and at most, from random samples
+// of the grid at the series stop and from the balls at the chains' starts.
+// "violations": of those four; "worst": the largest ratio.
+//
 // what = tie: a rebase test near its tie counts as tied at every size of delta that
 // the unscaled steps meet, as long as the bound is below 2^-23 |delta|.
 //
@@ -207,6 +212,88 @@ static int check_start(int samples, std::mt19937_64& g) {
   return bad ? 1 : 0;
 }
 
+// Steps from orbit index j to k (of z) in float-float, and exactly.
+static void step_to(const OrbitData& od, int j, int k, FF er_, FF ei_, FF& dr, FF& di, CL& exact) {
+  const CL eps((LD)er_.h + er_.l, (LD)ei_.h + ei_.l);
+  for (; j < k; j++) {
+    const FF zr = ff_from_double(od.z[j].x), zi = ff_from_double(od.z[j].y);
+    const FF tr = ff_add_twice_raw(zr.h, zr.l, dr), ti = ff_add_twice_raw(zi.h, zi.l, di);
+    FF nr, ni;
+    ff_cmul_add(tr, ti, dr, di, er_, ei_, nr, ni);
+    dr = nr;
+    di = ni;
+    // X[j - 1] is z[j]
+    const CL X((LD)od.xhi[j - 1].x + od.xlo[j - 1].x, (LD)od.xhi[j - 1].y + od.xlo[j - 1].y);
+    exact = (X + X + exact) * exact + eps;
+  }
+}
+
+struct Errors {
+  long n = 0;
+  LD sum = 0, most = 0;
+  void add(CL got, CL exact) {
+    const LD e = std::abs(got - exact) / std::abs(exact);
+    n++;
+    sum += e * e;
+    most = std::max(most, e);
+  }
+  LD rms() const { return sqrtl(sum / std::max(1L, n)); }
+};
+
+static int check_precision(const OrbitData& od, int samples, std::mt19937_64& g) {
+  std::uniform_real_distribution<double> U(0.0, 1.0);
+  Errors jump[2], steps[2];
+  for (int s = 0; s < samples; s++) {
+    const int chain = (int)(g() % kChains), i = (int)(g() % kChainClasses);
+    const JumpRec& r = tables.chain[(size_t)chain * kChainClasses + i];
+    if (tables.start_index[chain] < 0 || !(r.rho2 > 0)) continue;
+    const CL eps = eps_at(g() % er.size(), g() % ei.size());
+    const LD a = ldexpl(sqrtl(r.rho2) * (0.5L + 0.49L * U(g)), r.p), ph = 6.2831853L * U(g);
+    const CL gamma((LD)r.gamma.x + r.gamma.y, (LD)r.gamma.z + r.gamma.w);
+    FeState st = state(chain, CL(a * cosl(ph), a * sinl(ph)) - gamma * eps, eps, 0.0f);
+    FF dr = st.dr, di = st.di;
+    CL exact((LD)dr.h + dr.l, (LD)di.h + di.l);
+    const int j = st.j;
+    fe_chain_jump(view, st);
+    if (st.j == j) continue;
+    step_to(od, j, st.j, st.er, st.ei, dr, di, exact);
+    jump[0].add(CL((LD)st.dr.h + st.dr.l, (LD)st.di.h + st.di.l), exact);
+    steps[0].add(CL((LD)dr.h + dr.l, (LD)di.h + di.l), exact);
+  }
+  auto co = [](const CFE& x) { return CL(ldexpl(x.re, x.e), ldexpl(x.im, x.e)); };
+  for (int s = 0; s < samples; s++) {
+    const CL eps = eps_at(g() % er.size(), g() % ei.size());
+    const LD u = std::norm(eps);
+    int fire = 1, hi = od.xlen;
+    while (fire < hi) {
+      const int mid = (fire + hi) / 2;
+      const RFE& t = od.sa_min_fe[mid];
+      if (!std::isinf(t.m) && ldexpl(t.m, t.e) < u) hi = mid; else fire = mid + 1;
+    }
+    CFF d;
+    float bound = 0.0f;
+    int found = -1;
+    if (!fe_jump(view, fire, ffe(eps.real()), ffe(eps.imag()), d, bound, found)) continue;
+    const int f = std::max(1, fire - 3) - 1;
+    CL exact = (co(od.a_fe[f]) + (co(od.b_fe[f]) + co(od.c_fe[f]) * eps) * eps) * eps;
+    FF dr = ff(exact.real()), di = ff(exact.imag());
+    step_to(od, f + 1, found + 1, ff(eps.real()), ff(eps.imag()), dr, di, exact);
+    jump[1].add(CL(ldexpl((LD)d.re.h + d.re.l, d.e), ldexpl((LD)d.im.h + d.im.l, d.e)), exact);
+    steps[1].add(CL((LD)dr.h + dr.l, (LD)di.h + di.l), exact);
+  }
+  int bad = 0;
+  LD worst = 0;
+  for (int k = 0; k < 2; k++) {
+    const LD ratio[2] = {jump[k].rms() / steps[k].rms(), jump[k].most / steps[k].most};
+    for (LD q : ratio) {
+      worst = std::max(worst, q);
+      if (!(q <= 1)) bad++;
+    }
+  }
+  std::printf("%ld %d %.4f\n", std::min(jump[0].n, jump[1].n), bad, (double)worst);
+  return bad ? 1 : 0;
+}
+
 static int check_tie(int samples, std::mt19937_64& g) {
   std::uniform_real_distribution<double> U(0.0, 1.0);
   long bad = 0;
@@ -284,6 +371,7 @@ int main(int argc, char** argv) {
     view.jump_from[k] = tables.start_index[k] < 0 ? -1 : tables.start_index[k] + 1;
   if (!std::strcmp(what, "slope")) return check_slope(samples, g);
   if (!std::strcmp(what, "range")) return check_range(samples, g);
+  if (!std::strcmp(what, "precision")) return check_precision(od, samples, g);
   if (!std::strcmp(what, "start")) return check_start(samples, g);
   return 2;
 }

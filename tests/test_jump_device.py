@@ -72,3 +72,17 @@ def test_ties_of_the_rebase_test_at_every_size(run):
 def test_side_of_a_tie_is_the_fp64_path_s(run):
     ties, bad, decided = run("side", SEAHORSE, "1e-17", 37, 65, 1000, "center", samples=2000000)
     assert bad == "0" and int(ties) > 10000 and float(decided) > 0.5, (ties, bad, decided)
+
+
+# (eps above the float range: the float-float steps hold it unscaled)
+@pytest.mark.parametrize("where,step,nr,nc,N,mode", [
+    (SEAHORSE, "1.302083e-16", 4320, 7680, 50000, "probes"),
+    (SEAHORSE, "3e-17", 97, 131, 50000, "center"),
+    (17, "2e-20", 97, 131, 20000, "center"),
+    (20, "1e-23", 97, 131, 50000, "center"),
+    (25, "1e-28", 97, 131, 40000, "center"),
+    (28, "1e-31", 97, 131, 40000, "center"),
+])
+def test_jumps_are_as_near_as_the_steps(run, where, step, nr, nc, N, mode):
+    jumps, bad, worst = run("precision", where, step, nr, nc, N, mode, samples=1500)
+    assert bad == "0" and int(jumps) > 300, (jumps, bad, worst)
