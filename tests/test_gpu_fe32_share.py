@@ -26,3 +26,29 @@ def test_ties_of_the_rebase_test_are_decided(nm):
     share = m.stat(nm.STAT_FP64_REWORK) / (540 * 960)
     print("rework %.4f" % share)
     assert share <= 0.06
+
+
+# (view, the largest difference of the path without jumps)
+DEEP = ("-0.743643887037229095312187703165620156203167189531343718751406",
+        "0.131825904205267520317187749964062031515607811562296900001563")
+
+
+@pytest.mark.parametrize("view,bar", [
+    (dict(nr=1200, nc=1600, cre=C2["cre"], cim=C2["cim"], step="1.25e-16", N=20000), 4.82e-5),
+    (dict(nr=1080, nc=1920, cre=DEEP[0], cim=DEEP[1], step="5.208333333333333e-24", N=50000,
+          center=True), 2.83e-5),
+], ids=["2e-13", "1e-20"])
+def test_smoothing_is_as_near_as_without_jumps(nm, view, bar):
+    out = []
+    for path in (nm.PATH_FP64, nm.PATH_FE32):
+        m = setup_gpu(nm, dict(view, sc=1, tol=1e-10), path=path)
+        if view.get("center"):
+            m.set_option(nm.OPT_REFERENCE, nm.REFERENCE_CENTER)
+        m.precompute()
+        m.render()
+        out.append((m.grid()["iterations"].copy(), m.smoothing64().copy()))
+    (i0, s0), (i1, s1) = out
+    assert np.array_equal(i0, i1)
+    d = np.abs(s0 - s1).max()
+    print("largest difference %.3g" % d)
+    assert d <= bar
