@@ -7,7 +7,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
-#include <system_error>
 #include <thread>
 
 namespace nmg {
@@ -384,19 +383,11 @@ void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out, int*
 
 }  // namespace
 
-// The start jumps' records, and the orbit indexes at which classes ended near 0.
-static void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int threads,
-                              std::vector<JumpRec>& out, std::vector<int>& stops) {
-  JumpRec none{};
-  none.fire = -1;
-  none.rho2 = -1.0f;
-  out.assign((size_t)kJumpClasses * kJumpSubs, none);
-  if (od.xlen < 64 || !(eps_m > 0.0) || !std::isfinite(eps_m)) return;
-  // |eps| <= hi0 2^p, hi0 in [1/2, 1)
-  const int p = std::ilogb(eps_m) + 1 + eps_e;
+// The stop indexes in use, from the outermost samples inward, in units of 2^p with
+// |eps| <= hi0 2^p, hi0 in [1/2, 1).
+static std::vector<Start> starts_of(const OrbitData& od, double eps_m, int p) {
   const double hi0 = std::ldexp(eps_m, -(std::ilogb(eps_m) + 1));
-  // the stop indexes in use, from the outermost samples inward: fire = i for
-  // T_i < |eps|^2 <= T_{i-1}, T the prefix minima of the thresholds
+  // fire = i for T_i < |eps|^2 <= T_{i-1}, T the prefix minima of the thresholds
   auto radius = [&](int i) {  // sqrt(T_i) in units of 2^p (infinite: 4)
     const RFE& t = od.sa_min_fe[i];
     if (std::isinf(t.m)) return 4.0;
@@ -425,23 +416,13 @@ static void build_start_jumps(const OrbitData& od, double eps_m, int eps_e, int 
     above = r;
     i = lo;
   }
-  std::vector<int> stop(starts.size(), -1);
-  std::atomic<size_t> next{0};
-  auto work = [&] {
-    for (size_t k; (k = next.fetch_add(1)) < starts.size();)
-      build_class(od, starts[k], p, &out[k * kJumpSubs], &stop[k]);
-  };
-  const size_t nt = std::min(starts.size(), (size_t)std::max(1, threads));
-  std::vector<std::thread> pool;
-  try {
-    for (size_t t = 1; t < nt; t++) pool.emplace_back(work);
-  } catch (const std::system_error&) {  // no more threads: with those there are
-  }
-  work();
-  for (std::thread& t : pool) t.join();
-  stops = stop;
-  // the classes in use first: the device stops at the first unused one, and
-  // knows a class by its first record
+  return starts;
+}
+
+// The classes in use first: the device stops at the first unused one, and
+// knows a class by its first record.
+static void pack_starts(const std::vector<Start>& starts, std::vector<JumpRec>& out,
+                        const JumpRec& none) {
   size_t at = 0;
   for (size_t k = 0; k < starts.size(); k++) {
     JumpRec* r = &out[k * kJumpSubs];
@@ -655,41 +636,66 @@ EpsRange eps_range(const std::vector<RFE>& re, const std::vector<RFE>& im) {
   return r;
 }
 
+// work(0) .. work(n - 1) on at most `threads` threads, the caller's included.  work
+// throws nothing; a thread that cannot be had is done without.
+template <class Work>
+static void run_on(int threads, size_t n, const Work& work) {
+  std::atomic<size_t> next{0};
+  auto loop = [&] {
+    for (size_t k; (k = next.fetch_add(1)) < n;) work(k);
+  };
+  const size_t nt = std::min(n, (size_t)std::max(1, threads));
+  std::vector<std::thread> pool;
+  pool.reserve(nt);
+  try {
+    for (size_t t = 1; t < nt; t++) pool.emplace_back(loop);
+  } catch (...) {  // with those there are
+  }
+  loop();
+  for (std::thread& t : pool) t.join();
+}
+
 void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t) {
   JumpRec none{};
   none.rho2 = -1.0f;
   t.start_index.assign(kChains, -1);
-  std::vector<int> stops;
-  build_start_jumps(od, eps_m, eps_e, threads, t.start, stops);
   t.chain.assign((size_t)kChains * kChainClasses, none);
+  none.fire = -1;
+  t.start.assign((size_t)kJumpClasses * kJumpSubs, none);
   if (od.xlen < 64 || !(eps_m >= 0.0) || !std::isfinite(eps_m)) return;
   const double eps = eps_e < -1000 ? 0x1p-1000 : std::ldexp(eps_m, eps_e);
-  if (!(eps < 0x1p-16)) return;
-  // The chain from a rebase, and those from past the elements near 0 at which
-  // most start jumps (outermost samples first) and the rebase chain's end.
+  const bool chains = eps < 0x1p-16;
+  std::vector<Start> starts;
+  int p = 0;
+  if (eps_m > 0.0) {
+    p = std::ilogb(eps_m) + 1 + eps_e;
+    starts = starts_of(od, eps_m, p);
+  }
+  // the chain from a rebase, mostly the longest of these, then the start classes
+  std::vector<int> stops(starts.size(), -1);
+  int stop[kChains] = {-1, -1, -1};
+  const size_t first = chains ? 1 : 0;
+  run_on(threads, first + starts.size(), [&](size_t k) {
+    if (k < first)
+      build_chain(od, 0, eps, &t.chain[0], &stop[0]);
+    else
+      build_class(od, starts[k - first], p, &t.start[(k - first) * kJumpSubs], &stops[k - first]);
+  });
+  pack_starts(starts, t.start, none);
+  if (!chains) return;
+  // and the chains from past the elements near 0 at which most start jumps (outermost
+  // samples first) and the rebase chain's end
   std::vector<int> from{0};
-  auto add = [&](int stop) {
-    if (stop >= 0 && stop + 1 + 4 * kMinSteps < od.xlen && (int)from.size() < kChains &&
-        std::find(from.begin(), from.end(), stop + 1) == from.end())
-      from.push_back(stop + 1);
+  auto add = [&](int at) {
+    if (at >= 0 && at + 1 + 4 * kMinSteps < od.xlen && (int)from.size() < kChains &&
+        std::find(from.begin(), from.end(), at + 1) == from.end())
+      from.push_back(at + 1);
   };
   for (size_t k = 0; k < stops.size() && k < 2; k++) add(stops[k]);
-  std::vector<std::thread> pool;
-  int stop[kChains];
-  for (size_t k = 1; k < from.size(); k++) {
-    auto one = [&, k] { build_chain(od, from[k], eps, &t.chain[k * kChainClasses], &stop[k]); };
-    try {
-      pool.emplace_back(one);
-    } catch (const std::system_error&) {
-      one();
-    }
-  }
-  build_chain(od, 0, eps, &t.chain[0], &stop[0]);
-  for (std::thread& p : pool) p.join();
-  const size_t had = from.size();
   add(stop[0]);
-  for (size_t k = had; k < from.size(); k++)
-    build_chain(od, from[k], eps, &t.chain[k * kChainClasses], &stop[k]);
+  run_on(threads, from.size() - 1, [&](size_t k) {
+    build_chain(od, from[k + 1], eps, &t.chain[(k + 1) * kChainClasses], &stop[k + 1]);
+  });
   for (size_t k = 0; k < from.size(); k++) t.start_index[k] = from[k];
 }
 

@@ -86,3 +86,20 @@ def test_side_of_a_tie_is_the_fp64_path_s(run):
 def test_jumps_are_as_near_as_the_steps(run, where, step, nr, nc, N, mode):
     jumps, bad, worst = run("precision", where, step, nr, nc, N, mode, samples=1500)
     assert bad == "0" and int(jumps) > 300, (jumps, bad, worst)
+
+
+@pytest.mark.parametrize("where,step,N", [(SEAHORSE, "1e-16", 50000), (20, "1e-22", 20000),
+                                          (40, "1e-43", 60000)])
+def test_tables_keep_to_their_threads(tmp_path, where, step, N):
+    if not shutil.which("g++"):
+        pytest.skip("no g++")
+    exe = str(tmp_path / "jump_threads")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-pthread", "-I", CSRC,
+                    "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
+                    os.path.join(HERE, "native", "jump_threads.cpp"),
+                    os.path.join(CSRC, "jump.cpp"), os.path.join(CSRC, "mpview.cpp"),
+                    "-o", exe, "-l:libgmp.so.10", "-ldl"], check=True)
+    re, im = where if isinstance(where, tuple) else center(where)
+    out = subprocess.run([exe, re, im, step, "97", "131", str(N)], capture_output=True, text=True)
+    differ, beyond, started = out.stdout.split()
+    assert differ == "0" and beyond == "0" and int(started) > 0, out.stdout
