@@ -142,6 +142,40 @@ int ensure_coords(nm_handle* h) {
   return NM_OK;
 }
 
+int host_threads(const nm_handle* h) {
+  return h->threads > 0 ? h->threads : (int)std::thread::hardware_concurrency();
+}
+
+// The FP32 path's jumps (jump.hpp), for |eps| up to the farthest sample's; true when
+// they were built: the handle renders by that path, from tables of its own that have
+// none yet.  Where they would not pay for themselves (build_jumps) there are none.
+bool ensure_jumps(nm_handle* h) {
+  if (h->path != NM_PATH_FE32 || !h->precomputed || h->orbit_src || h->od.double_loop ||
+      h->jump_tried)
+    return false;
+  h->jump_tried = true;
+  const nmg::EpsRange range = h->od.sa_fp64_ok ? nmg::eps_range(h->eps_re, h->eps_im)
+                                               : nmg::eps_range(h->eps_re_fe, h->eps_im_fe);
+  nmg::JumpTables t;
+  nmg::build_jumps(h->od, range.norm(), range.e, host_threads(h), t,
+                   (long long)h->view.rows() * h->view.cols());
+  const bool any = t.start[0].fire >= 0 || t.start_index[0] >= 0;
+  if (!any) return false;
+  h->jump = std::move(t.start);
+  h->jump.insert(h->jump.end(), t.chain.begin(), t.chain.end());
+  h->jump_er = range.re_limit();
+  h->jump_ei = range.im_limit();
+  h->jump_x2 = 0.0f;
+  for (int k = 0; k < nmg::kChains; k++) {
+    // X[s] is z[s + 1]
+    h->jump_from[k] = t.start_index[k] < 0 ? -1 : t.start_index[k] + 1;
+    for (int i = 0; i < nmg::kChainClasses; i++)
+      if (t.chain[(size_t)k * nmg::kChainClasses + i].rho2 > 0.0f)
+        h->jump_x2 = std::max(h->jump_x2, (float)std::exp2(-nmg::kChainTop - 2 * i));
+  }
+  return true;
+}
+
 int do_upload(nm_handle* h) {
   int rc;
   if ((rc = ensure_device(h))) return rc;
@@ -156,6 +190,7 @@ int do_upload(nm_handle* h) {
   if (h->orbit_src && !h->orbit_src->uploaded)
     if ((rc = do_upload(h->orbit_src))) return rc;
   const bool own = h->orbit_src == nullptr;
+  ensure_jumps(h);
   if (own && h->precomputed && !h->od.xmp.empty())
     if ((rc = upload(h->d_x_mp, h->od.xmp, h->stream))) return rc;
   if (h->precomputed) {
@@ -277,26 +312,6 @@ void build_front32_tables(nm_handle* h, bool series = true) {
   }
 }
 
-// The FP32 path's jumps (jump.hpp), for |eps| up to the farthest sample's.
-void build_jump_tables(nm_handle* h, int threads) {
-  const nmg::EpsRange range = h->od.sa_fp64_ok ? nmg::eps_range(h->eps_re, h->eps_im)
-                                               : nmg::eps_range(h->eps_re_fe, h->eps_im_fe);
-  nmg::JumpTables t;
-  nmg::build_jumps(h->od, range.norm(), range.e, threads, t);
-  h->jump = std::move(t.start);
-  h->jump.insert(h->jump.end(), t.chain.begin(), t.chain.end());
-  h->jump_er = range.re_limit();
-  h->jump_ei = range.im_limit();
-  h->jump_x2 = 0.0f;
-  for (int k = 0; k < nmg::kChains; k++) {
-    // X[s] is z[s + 1]
-    h->jump_from[k] = t.start_index[k] < 0 ? -1 : t.start_index[k] + 1;
-    for (int i = 0; i < nmg::kChainClasses; i++)
-      if (t.chain[(size_t)k * nmg::kChainClasses + i].rho2 > 0.0f)
-        h->jump_x2 = std::max(h->jump_x2, (float)std::exp2(-nmg::kChainTop - 2 * i));
-  }
-}
-
 int check_handle(const nm_handle* h) {
   if (!h) return fail(NM_ERR_ARG, "null handle");
   return NM_OK;
@@ -313,11 +328,13 @@ void set_fe_tables(const nm_handle* h, nmg::DeviceView& v) {
     v.sa_b32 = t->d_b32.p;
     v.sa_c32 = t->d_c32.p;
     v.sa_min32 = t->d_sa_min32.p;
-    v.jump = t->jump.empty() ? nullptr : t->d_jump.p;
-    std::copy(t->jump_from, t->jump_from + nmg::kChains, v.jump_from);
-    v.jump_x2 = t->jump_x2;
-    v.jump_er = t->jump_er;
-    v.jump_ei = t->jump_ei;
+    if (!t->jump.empty()) {  // else none: jump_x2 0
+      v.jump = t->d_jump.p;
+      std::copy(t->jump_from, t->jump_from + nmg::kChains, v.jump_from);
+      v.jump_x2 = t->jump_x2;
+      v.jump_er = t->jump_er;
+      v.jump_ei = t->jump_ei;
+    }
   }
   v.sa_fe = h->od.sa_fp64_ok ? 0 : 1;
   if (!v.sa_fe) return;
@@ -355,8 +372,15 @@ int nmg::prepare_view(nm_handle* h, int r0, int r1, nmg::DeviceView& v, nmg::Ker
                               "nm_precompute again after changing the path");
   if (int rc = ensure_grid(h)) return rc;
   if (int rc = ensure_coords(h)) return rc;
-  if (!h->uploaded)
+  if (!h->uploaded) {
     if (int rc = do_upload(h)) return rc;
+  } else if (ensure_jumps(h)) {  // uploaded while the handle took another path
+    h->uploaded = false;
+    if (int rc = upload(h->d_jump, h->jump, h->stream)) return rc;
+    NM_CUDA(cudaStreamSynchronize(h->stream));
+    h->uploaded = true;
+    h->generation++;
+  }
   std::memset(&v, 0, sizeof v);
   v.nr = nr;
   v.nc = nc;
@@ -467,6 +491,7 @@ nm_handle* nm_copy(const nm_handle* src) {
   h->c32 = src->c32;
   h->sa_min32 = src->sa_min32;
   h->jump = src->jump;
+  h->jump_tried = src->jump_tried;
   std::copy(src->jump_from, src->jump_from + nmg::kChains, h->jump_from);
   h->jump_x2 = src->jump_x2;
   h->jump_er = src->jump_er;
@@ -712,6 +737,8 @@ int nm_precompute(nm_handle* h) {
   h->coords_valid = false;
   if (int rc = ensure_coords(h)) return rc;
   h->precomputed = false;
+  h->jump_tried = false;
+  h->jump.clear();
   h->orbit_src = nullptr;  // from here on the handle's own orbit
   h->od_zlen = 0;
   h->tables_stamp++;  // previews sharing the old orbit no longer render
@@ -729,15 +756,14 @@ int nm_precompute(nm_handle* h) {
     h->precomputed = true;
   } else if (!h->view.use_hardware() ||
              (h->path != NM_PATH_REFERENCE && h->path != NM_PATH_MP)) {
-    int threads = h->threads > 0 ? h->threads : (int)std::thread::hardware_concurrency();
-    if (h->view.precompute(threads, h->od, h->reference_mode, h->path == NM_PATH_MP,
+    if (h->view.precompute(host_threads(h), h->od, h->reference_mode, h->path == NM_PATH_MP,
                            gpu_probe_lengths, h))
       return fail(NM_ERR_STATE, "precompute failed");
     h->view.eps_tables(h->od, h->eps_re, h->eps_im);
     if (!h->od.sa_fp64_ok) h->view.eps_tables_fe(h->eps_re_fe, h->eps_im_fe);
     build_front32_tables(h);
-    build_jump_tables(h, threads);
     h->precomputed = true;
+    ensure_jumps(h);
   }
   h->precompute_us =
       std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count();

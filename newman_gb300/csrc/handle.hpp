@@ -117,7 +117,8 @@ struct nm_handle {
   std::vector<nmg::FFE> eps32_re, eps32_im;
   std::vector<nmg::CFFE> a32, b32, c32;
   std::vector<nmg::TFE> sa_min32;
-  std::vector<nmg::JumpRec> jump;
+  std::vector<nmg::JumpRec> jump;  // empty: none (yet)
+  bool jump_tried = false;         // for the current orbit and series
   int32_t jump_from[nmg::kChains] = {};
   float jump_x2 = 0.0f, jump_er = 0.0f, jump_ei = 0.0f;
   DevBuf<nmg::FFE> d_eps32_re, d_eps32_im;

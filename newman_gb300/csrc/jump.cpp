@@ -1,6 +1,6 @@
 // The polynomials of jump.hpp, on the host in double.
 #if defined(__GNUC__)
-#pragma GCC optimize("O3")
+#pragma GCC optimize("O3", "no-math-errno")  // (square roots in vectors)
 #endif
 #include "jump.hpp"
 
@@ -150,59 +150,47 @@ bool make_record(const Poly<NB>& u, int fire, int n, int p, double rho, double q
   return true;
 }
 
-// Adds order c times order b - c of u to order b of its square: the terms kept
-// to (sr, si), the magnitudes of those beyond the degree to w.
+// Adds order c times order b - c of u to order b of its square, the terms kept.
 template <int b, int c, int NB>
-inline void add_product(const Poly<NB>& u, const double (*a)[D + 1], double* sr, double* si,
-                        double* w) {
+inline void add_product(const Poly<NB>& u, double* sr, double* si) {
   constexpr int m = kTerms[c], n = kTerms[b - c], keep = kTerms[b];
   constexpr bool square = 2 * c == b;
-  const double *yr = u.re[b - c], *yi = u.im[b - c], *ya = a[b - c];
+  const double *yr = u.re[b - c], *yi = u.im[b - c];
   for (int i = 0; i < m; i++) {
     // a square's pairs once: j >= i
     const int lo = square ? i : 0, mid = std::min(n, std::max(lo, keep - i));
-    const double xr = 2.0 * u.re[c][i], xi = 2.0 * u.im[c][i], xa = 2.0 * a[c][i];
+    const double xr = 2.0 * u.re[c][i], xi = 2.0 * u.im[c][i];
     for (int j = lo; j < mid; j++) {
       sr[i + j] += xr * yr[j] - xi * yi[j];
       si[i + j] += xr * yi[j] + xi * yr[j];
     }
-    for (int j = mid; j < n; j++) w[i + j] += xa * ya[j];
-    if (square) {  // and the diagonal half
-      if (2 * i < keep) {
-        sr[2 * i] -= 0.5 * (xr * yr[i] - xi * yi[i]);
-        si[2 * i] -= 0.5 * (xr * yi[i] + xi * yr[i]);
-      } else {
-        w[2 * i] -= 0.5 * xa * ya[i];
-      }
+    if (square && 2 * i < keep) {  // and the diagonal half
+      sr[2 * i] -= 0.5 * (xr * yr[i] - xi * yi[i]);
+      si[2 * i] -= 0.5 * (xr * yi[i] + xi * yr[i]);
     }
   }
-  if constexpr (2 * (c + 1) <= b) add_product<b, c + 1>(u, a, sr, si, w);
+  if constexpr (2 * (c + 1) <= b) add_product<b, c + 1>(u, sr, si);
 }
 
 // One step, u' = 2 X u + F (u^2) + eps (eps_x: of order 0's x, as start jumps
-// have it; else of order 1's constant), over orders [0, nb), and the sums
-// |u_i| |u_j| beyond the degree by order and degree (a: the coefficients'
-// magnitudes).
+// have it; else of order 1's constant), over orders [0, nb).
 template <int b, int NB>
-inline void step_order(const Poly<NB>& u, int nb, const double (*a)[D + 1], double xr, double xi,
-                       double F, Poly<NB>& o, double (*w)[2 * D + 2]) {
+inline void step_order(const Poly<NB>& u, int nb, double xr, double xi, double F, Poly<NB>& o) {
   double sr[D + 1] = {}, si[D + 1] = {};
-  std::fill(w[b], w[b] + 2 * D + 2, 0.0);
-  add_product<b, 0>(u, a, sr, si, w[b]);
+  add_product<b, 0>(u, sr, si);
   for (int k = 0; k < kTerms[b]; k++) {
     o.re[b][k] = 2.0 * (xr * u.re[b][k] - xi * u.im[b][k]) + F * sr[k];
     o.im[b][k] = 2.0 * (xr * u.im[b][k] + xi * u.re[b][k]) + F * si[k];
   }
   if constexpr (b + 1 < NB) {
-    if (b + 1 < nb) step_order<b + 1>(u, nb, a, xr, xi, F, o, w);
+    if (b + 1 < nb) step_order<b + 1>(u, nb, xr, xi, F, o);
   }
 }
 template <int NB>
-void step_poly(Poly<NB>& u, int nb, const double (*a)[D + 1], double xr, double xi, double F,
-               double eps_x, double (*w)[2 * D + 2]) {
+void step_poly(Poly<NB>& u, int nb, double xr, double xi, double F, double eps_x) {
   Poly<NB> o;
   o.s = u.s;
-  step_order<0>(u, nb, a, xr, xi, F, o, w);
+  step_order<0>(u, nb, xr, xi, F, o);
   o.re[0][1] += eps_x;
   if constexpr (NB > 1) {
     if (nb > 1) o.re[1][0] += 1.0;
@@ -212,6 +200,41 @@ void step_poly(Poly<NB>& u, int nb, const double (*a)[D + 1], double xr, double 
     }
   }
   u = o;
+}
+
+// What a square drops at radius rho, out[b] = the sum over the pairs of order b's
+// terms |u_i| |u_j| rho^(i + j) beyond its degree (a: the coefficients' magnitudes).
+// At a radius t rho, t <= 1, it is at most t^kTerms[b] of that: the least power it
+// has.  (The sums by degree, taken at each radius, cost as much again as the step.)
+template <int NB>
+void dropped_by_square(const double (*a)[D + 1], int nb, double rho, double* out) {
+  double A[NB][D + 1], S[NB][D + 2];
+  for (int b = 0; b < nb; b++) {
+    double p = 1.0;
+    for (int k = 0; k < kTerms[b]; k++) {
+      A[b][k] = a[b][k] * p;
+      p *= rho;
+    }
+    S[b][kTerms[b]] = 0.0;
+    for (int k = kTerms[b] - 1; k >= 0; k--) S[b][k] = S[b][k + 1] + A[b][k];
+  }
+  for (int b = 0; b < nb; b++) {
+    double sum = 0.0;
+    for (int c = 0; c <= b; c++)
+      for (int i = 0; i < kTerms[c]; i++) {
+        const int j = std::max(0, kTerms[b] - i);
+        if (j < kTerms[b - c]) sum += A[c][i] * S[b - c][j];
+      }
+    out[b] = sum;
+  }
+}
+
+// x^n for the numbers of terms.
+double power(double x, int n) {
+  double p = 1.0;
+  for (; n; n >>= 1, x *= x)
+    if (n & 1) p *= x;
+  return p;
 }
 
 // With x' = x + theta eps, theta = the constant of order 1 over the linear
@@ -291,6 +314,12 @@ struct Start {
   double hi, lo;  // |eps| of the class's samples, in units of 2^p: (lo, hi]
 };
 
+// The radii of a class's records: steps of 2^-1/4 to half, then octaves.
+double sub_radius(double hi, int i) {
+  for (int k = 0; k < i; k++) hi *= k < 4 ? 0.84089641525371461 : 0.5;
+  return hi;
+}
+
 void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out, int* stop) {
   *stop = -1;
   const int f = std::max(1, st.fire - 3) - 1;
@@ -307,31 +336,30 @@ void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out, int*
       u.im[0][k] = e < -1000 ? 0.0 : std::ldexp(t[k - 1].im, e);
     }
   }
-  double a[1][D + 1] = {}, w[1][2 * D + 2];
+  double a[1][D + 1] = {};
   for (int k = 1; k <= 3; k++) a[0][k] = norm(u.re[0][k], u.im[0][k]);
   if (!(a[0][1] > 0.0)) return;
   double rho[kJumpSubs], R[kJumpSubs], Q[kJumpSubs], P[kJumpSubs];
   bool alive[kJumpSubs];
-  double x = st.hi;
   for (int i = 0; i < kJumpSubs; i++) {
-    rho[i] = x;
-    alive[i] = x > 0.0 && (i == 0 || x > st.lo);
-    x *= i < 4 ? 0.84089641525371461 : 0.5;  // 2^-1/4, then octaves
+    rho[i] = sub_radius(st.hi, i);
+    alive[i] = rho[i] > 0.0 && (i == 0 || rho[i] > st.lo);
     R[i] = P[i] = 0.0;
     // the FP64 path's rounding of its start
     Q[i] = 0x1p-49 * sum_pow(a[0], 1, 3, rho[i]);
   }
   Poly<1> prev = u;
-  double prev_q[kJumpSubs] = {};
+  double prev_q[kJumpSubs] = {}, fall[kJumpSubs] = {};  // (rho[i] / rho[top])^kTerms[0]
+  int top = -1;
   for (int n = f; n <= last; n++) {
     if (u.s < -900) return;  // the products below would leave the double range
     const double xr = od.xhi[n].x, xi = od.xhi[n].y, xm = norm(xr, xi) * (1.0 + 0x1p-50);
     const double F = pow2(u.s);
     for (int k = 1; k <= D; k++) a[0][k] = norm(u.re[0][k], u.im[0][k]);
     bool any = false;
+    sums_pow(a[0], 1, D, rho, kJumpSubs, P);
     for (int i = 0; i < kJumpSubs; i++) {
       if (!alive[i]) continue;
-      P[i] = sum_pow(a[0], 1, D, rho[i]);
       const double dmax = (P[i] + R[i] + Q[i]) * F;
       // the FP64 path has this sample at the same orbit index: it does not
       // rebase while |delta| < |X| - |delta|, nor bail out below 1000
@@ -350,10 +378,16 @@ void build_class(const OrbitData& od, const Start& st, int p, JumpRec* out, int*
     prev = u;
     std::copy(Q, Q + kJumpSubs, prev_q);
     const double eps = pow2(p - u.s);  // eps = x 2^p
-    step_poly(u, 1, a, xr, xi, F, eps, w);
+    step_poly(u, 1, xr, xi, F, eps);
+    if (top < 0 || !alive[top]) {
+      for (top = 0; !alive[top];) top++;
+      for (int i = top; i < kJumpSubs; i++) fall[i] = power(rho[i] / rho[top], kTerms[0]);
+    }
+    double drop = 0.0;
+    dropped_by_square<1>(a, 1, rho[top], &drop);
     for (int i = 0; i < kJumpSubs; i++) {
       if (!alive[i]) continue;
-      const double h = F * sum_pow(w[0], D + 1, 2 * D, rho[i]);
+      const double h = F * drop * fall[i];
       // R: (p + R)^2 = p^2 + (2p + R) R, and p^2's terms beyond the degree
       R[i] = (2.0 * xm + F * (2.0 * P[i] + R[i])) * R[i] + h;
       // Q adds, a step: the FP64 path's rounding and its truncated orbit,
@@ -419,6 +453,23 @@ static std::vector<Start> starts_of(const OrbitData& od, double eps_m, int p) {
   return starts;
 }
 
+// The mean of the steps that start jumps save over |eps| <= hi0 2^p.
+static double mean_steps(const std::vector<Start>& starts, const std::vector<JumpRec>& recs,
+                         double hi0) {
+  double sum = 0.0;
+  for (size_t k = 0; k < starts.size(); k++) {
+    const int f = std::max(1, starts[k].fire - 3) - 1;
+    double x = starts[k].hi;
+    for (int i = 0; i < kJumpSubs; i++) {
+      const double in = i + 1 < kJumpSubs ? sub_radius(starts[k].hi, i + 1) : starts[k].lo;
+      const double y = std::max(starts[k].lo, std::min(x, in));
+      if (recs[k * kJumpSubs + i].rho2 > 0.0f) sum += (x * x - y * y) * (recs[k * kJumpSubs + i].n - f);
+      x = y;
+    }
+  }
+  return sum / (hi0 * hi0);
+}
+
 // The classes in use first: the device stops at the first unused one, and
 // knows a class by its first record.
 static void pack_starts(const std::vector<Start>& starts, std::vector<JumpRec>& out,
@@ -456,10 +507,12 @@ void build_chain(const OrbitData& od, int s, double eps, JumpRec* out, int* stop
   }
   Poly<B> u{};
   u.re[0][1] = 1.0;
-  double rho[C], R[C], Q[C], P[C], E[C], S[C], H[C], T[C], order[B][C], power[2 * B];
+  double rho[C], R[C], Q[C], P[C], E[C], S[C], T[C], order[B][C], epow[2 * B];
+  double fall[B][C];  // (rho[i] / rho[first])^kTerms[b]
+  int fall_of = -1;   // first, as those were taken
   bool alive[C], open[C];
-  power[0] = 1.0;
-  for (int b = 1; b < 2 * B; b++) power[b] = power[b - 1] * eps;
+  epow[0] = 1.0;
+  for (int b = 1; b < 2 * B; b++) epow[b] = epow[b - 1] * eps;
   for (int i = 0; i < C; i++) {
     rho[i] = std::exp2(-0.5 * kChainTop - i);
     R[i] = P[i] = E[i] = 0.0;
@@ -471,7 +524,7 @@ void build_chain(const OrbitData& od, int s, double eps, JumpRec* out, int* stop
   double gr = 0.0, gi = 0.0;  // Gamma: x = delta_s + Gamma eps
   Poly<B> prev = u;
   double prev_q[C] = {}, prev_rho[C] = {}, prev_g[2] = {};
-  double a[B][D + 1] = {}, w[B][2 * D + 2];
+  double a[B][D + 1] = {};
   Shift shift;
   int stops[C], nstops = 0;
   for (int n = s; n <= last; n++) {
@@ -555,26 +608,27 @@ void build_chain(const OrbitData& od, int s, double eps, JumpRec* out, int* stop
     std::copy(rho, rho + C, prev_rho);
     prev_g[0] = gr;
     prev_g[1] = gi;
-    step_poly(u, nb, a, xr, xi, 1.0, 0.0, w);
-    // the square's terms beyond the degrees (order b's scale with a ball's radius
-    // to the kTerms[b] at least) and beyond the orders
-    sums_pow(w[0], D + 1, 2 * D, rho + first, full, H + first);
-    for (int i = first; i <= lin; i++) T[i] = 0.0;
-    for (int b = nb - 1; b >= 1; b--) {
-      sums_pow(w[b], kTerms[b], 2 * D, rho + first, full, S + first);
-      for (int i = first; i <= lin; i++) T[i] = (T[i] + S[i]) * eps;
+    step_poly(u, nb, xr, xi, 1.0, 0.0);
+    // the square's terms beyond the degrees and beyond the orders
+    while (first < C && !alive[first]) first++;
+    if (fall_of != first) {
+      fall_of = first;
+      for (int i = first; i < C; i++)
+        for (int b = 0; b < nb; b++) fall[b][i] = power(rho[i] / rho[first], kTerms[b]);
     }
-    for (int i = first; i <= lin; i++) {
+    double drop[B];
+    dropped_by_square<B>(a, nb, rho[first], drop);
+    for (int b = 1; b < nb; b++) drop[b] *= epow[b];
+    for (int i = std::min(first, lin); i <= lin; i++) {
       double x = nb == 1 ? eps : 0.0;
       for (int b = 1; b < nb; b++)
-        for (int c = nb - b; c < nb; c++) x += order[b][i] * order[c][i] * power[b + c];
-      H[i] += T[i];
+        for (int c = nb - b; c < nb; c++) x += order[b][i] * order[c][i] * epow[b + c];
       T[i] = x;
     }
     for (int i = 0; i < C; i++) {
       if (!alive[i]) continue;
-      const double t = i > lin ? rho[i] / rho[lin] : 1.0;
-      const double h = i > lin ? H[lin] * t * t + T[lin] : H[i] + T[i];
+      double h = T[std::min(i, lin)];
+      for (int b = 0; b < nb; b++) h += drop[b] * fall[b][i];
       const double d = P[i] + E[i];
       R[i] = (2.0 * xm + 2.0 * d + R[i]) * R[i] + h;
       // as build_class, with eps's own terms
@@ -600,6 +654,7 @@ void build_chain(const OrbitData& od, int s, double eps, JumpRec* out, int* stop
       R[i] += r;
       Q[i] += r + shift.rounding(rho[i], eps);
       rho[i] -= shift.tm * eps;
+      fall_of = -1;
       // (see Shift::dropped), and half of it in all
       if (rho[i] < 0.5 * std::exp2(-0.5 * kChainTop - i) || shift.tm * eps > 0x1p-5 * rho[i])
         alive[i] = false;
@@ -655,13 +710,34 @@ static void run_on(int threads, size_t n, const Work& work) {
   for (std::thread& t : pool) t.join();
 }
 
-void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t) {
+// Where tables are built, by what a first render of a new view gains less the build
+// (2-3 ms on 16 threads for most views; precompute and render together, without -> with,
+// on nine views at widths from 1e-13 to 1e-120, and in brackets later renders):
+// * grids of 500,000 samples and more: 960x540 at 1e-15 9.2 -> 9.9 ms (7.3 -> 5.4), at
+//   3e-17 29.7 -> 30.4 (24.3 -> 22.0), at 2e-13 32.5 -> 32.4, at 1e-20 32.8 -> 29.0;
+//   1280x720 from 13.2 -> 12.4 at 1e-15 to 39.8 -> 31.4 at 1e-20;
+// * from 2^17 on where the start jumps alone save 0.42e9 steps in all: 517x333 at 1e-20
+//   27.5 -> 27.0 (12.4 -> 10.4), at 1e-25 37.4 -> 37.0 (14.6 -> 11.7); at 1e-15, where
+//   they do not, it was 7.6 -> 9.9 (5.9 -> 5.4).  That is known only once they are
+//   built (1.3 ms in vain at 1e-15), so first the stop index, which they rarely pass,
+//   has to allow it;
+// * never on smaller grids: 320x240 at 1e-20 24.7 -> 26.2, at 1e-15 6.7 -> 9.4;
+// * and nowhere that no sample stops the series: all end about where the reference
+//   orbit does (the frames below 1e-16 of a zoom into a center of 15 digits).
+constexpr long long kJumpSamples = 500000, kJumpFewSamples = 1 << 17;
+constexpr double kJumpStopSteps = 0.7e9, kJumpStartSteps = 0.42e9;
+
+void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t,
+                 long long samples) {
   JumpRec none{};
-  none.rho2 = -1.0f;
-  t.start_index.assign(kChains, -1);
-  t.chain.assign((size_t)kChains * kChainClasses, none);
   none.fire = -1;
-  t.start.assign((size_t)kJumpClasses * kJumpSubs, none);
+  none.rho2 = -1.0f;
+  auto clear = [&] {
+    t.start.assign((size_t)kJumpClasses * kJumpSubs, none);
+    t.chain.assign((size_t)kChains * kChainClasses, none);
+    t.start_index.assign(kChains, -1);
+  };
+  clear();
   if (od.xlen < 64 || !(eps_m >= 0.0) || !std::isfinite(eps_m)) return;
   const double eps = eps_e < -1000 ? 0x1p-1000 : std::ldexp(eps_m, eps_e);
   const bool chains = eps < 0x1p-16;
@@ -671,6 +747,10 @@ void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, Jump
     p = std::ilogb(eps_m) + 1 + eps_e;
     starts = starts_of(od, eps_m, p);
   }
+  const bool few = samples < kJumpSamples;
+  if (starts.empty() || samples < kJumpFewSamples ||
+      (few && (double)samples * starts[0].fire < kJumpStopSteps))
+    return;
   // the chain from a rebase, mostly the longest of these, then the start classes
   std::vector<int> stops(starts.size(), -1);
   int stop[kChains] = {-1, -1, -1};
@@ -681,6 +761,11 @@ void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, Jump
     else
       build_class(od, starts[k - first], p, &t.start[(k - first) * kJumpSubs], &stops[k - first]);
   });
+  t.start_steps = mean_steps(starts, t.start, std::ldexp(eps_m, -(std::ilogb(eps_m) + 1)));
+  if (few && (double)samples * t.start_steps < kJumpStartSteps) {
+    clear();
+    return;
+  }
   pack_starts(starts, t.start, none);
   if (!chains) return;
   // and the chains from past the elements near 0 at which most start jumps (outermost

@@ -47,6 +47,7 @@ struct JumpTables {
   std::vector<JumpRec> chain;    // kChains * kChainClasses (class i: |x|^2 <
                                  // 2^-(kChainTop + 2 i)); unused: rho2 -1
   std::vector<int> start_index;  // kChains: X index each starts at; -1: none
+  double start_steps = 0.0;      // that start jumps save, the mean over the disk of |eps|
 };
 
 // The largest |component|s of a grid's eps: re 2^e and im 2^e.
@@ -61,7 +62,10 @@ struct EpsRange {
 EpsRange eps_range(const std::vector<double>& re, const std::vector<double>& im);
 EpsRange eps_range(const std::vector<RFE>& re, const std::vector<RFE>& im);
 
-// The tables of a precomputed deep view whose samples have |eps| <= m 2^e.
-void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t);
+// The tables of a precomputed deep view whose `samples` samples have |eps| <= m 2^e,
+// on at most `threads` threads; unused throughout where they would not pay for
+// themselves in one render (kJumpSamples).
+void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, JumpTables& t,
+                 long long samples = 1ll << 62);
 
 }  // namespace nmg

@@ -18,6 +18,9 @@
 // of the grid at the series stop and from the balls at the chains' starts.
 // "violations": of those four; "worst": the largest ratio.
 //
+// what = sizes: prints for grids of 2^17 - 1, 2^17, 499,999 and 500,000 samples whether
+// they have tables (1) or none (0), as one number.
+//
 // what = tie: a rebase test near its tie counts as tied at every size of delta that
 // the unscaled steps meet, as long as the bound is below 2^-23 |delta|.
 //
@@ -359,6 +362,18 @@ int main(int argc, char** argv) {
     return 4;
   v.eps_tables_fe(er, ei);
   range = eps_range(er, ei);
+  if (!std::strcmp(what, "sizes")) {
+    for (long long n : {(1ll << 17) - 1, 1ll << 17, 499999ll, 500000ll}) {
+      JumpTables t;
+      build_jumps(od, range.norm(), range.e, 4, t, n);
+      bool any = t.start[0].fire >= 0;
+      for (int k = 0; k < kChains; k++) any |= t.start_index[k] >= 0;
+      for (const JumpRec& r : t.chain) any |= r.rho2 > 0;
+      std::printf("%d", any);
+    }
+    std::printf(" 0 0\n");
+    return 0;
+  }
   build_jumps(od, range.norm(), range.e, 4, tables);
   records = tables.start;
   records.insert(records.end(), tables.chain.begin(), tables.chain.end());

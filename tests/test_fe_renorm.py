@@ -16,15 +16,20 @@ CUDA_INC = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include
 WALK = json.load(open(os.path.join(HERE, "golden", "deep_centers.json")))["steps"]
 
 
-@pytest.mark.parametrize("width,step", [("1e-30", "1e-31"), ("1e-45", "1e-47")])
-def test_pieces_do_not_change_the_state(tmp_path, width, step):
+@pytest.fixture(scope="module")
+def exe(tmp_path_factory):
     if not shutil.which("g++"):
         pytest.skip("no g++")
-    exe = str(tmp_path / "fe_renorm")
+    path = str(tmp_path_factory.mktemp("renorm") / "fe_renorm")
     subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-pthread", "-I", CSRC,
                     "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
                     os.path.join(HERE, "native", "fe_renorm.cpp"),
-                    os.path.join(CSRC, "mpview.cpp"), "-o", exe, "-l:libgmp.so.10"], check=True)
+                    os.path.join(CSRC, "mpview.cpp"), "-o", path, "-l:libgmp.so.10"], check=True)
+    return path
+
+
+@pytest.mark.parametrize("width,step", [("1e-30", "1e-31"), ("1e-45", "1e-47")])
+def test_pieces_do_not_change_the_state(exe, width, step):
     at = WALK[next(i for i, s in enumerate(WALK) if Decimal(s["width"]) <= Decimal(width)) - 1]
     out = subprocess.run([exe, at["next_center_re"], at["next_center_im"], step, "48", "64",
                           "20000", "400", "19990", "3"], capture_output=True, text=True)

@@ -10,16 +10,26 @@ import pytest
 from test_jumps import CSRC, CUDA_INC, HERE, ROOT, SEAHORSE, center
 
 
-@pytest.fixture(scope="module")
-def run(tmp_path_factory):
+def compiled(tmp_path_factory, name):
     if not shutil.which("g++"):
         pytest.skip("no g++")
-    exe = str(tmp_path_factory.mktemp("jump_device") / "jump_device")
+    exe = str(tmp_path_factory.mktemp(name) / name)
     subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-pthread", "-I", CSRC,
                     "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
-                    os.path.join(HERE, "native", "jump_device.cpp"),
+                    os.path.join(HERE, "native", name + ".cpp"),
                     os.path.join(CSRC, "jump.cpp"), os.path.join(CSRC, "mpview.cpp"),
-                    "-o", exe, "-l:libgmp.so.10"], check=True)
+                    "-o", exe, "-l:libgmp.so.10", "-ldl"], check=True)
+    return exe
+
+
+@pytest.fixture(scope="module")
+def threads(tmp_path_factory):
+    return compiled(tmp_path_factory, "jump_threads")
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    exe = compiled(tmp_path_factory, "jump_device")
 
     def go(what, where, step, nr, nc, N, mode, samples=20000, seed=5):
         re, im = where if isinstance(where, tuple) else center(where)
@@ -90,16 +100,20 @@ def test_jumps_are_as_near_as_the_steps(run, where, step, nr, nc, N, mode):
 
 @pytest.mark.parametrize("where,step,N", [(SEAHORSE, "1e-16", 50000), (20, "1e-22", 20000),
                                           (40, "1e-43", 60000)])
-def test_tables_keep_to_their_threads(tmp_path, where, step, N):
-    if not shutil.which("g++"):
-        pytest.skip("no g++")
-    exe = str(tmp_path / "jump_threads")
-    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-pthread", "-I", CSRC,
-                    "-I", os.path.join(ROOT, "include"), "-I", CUDA_INC,
-                    os.path.join(HERE, "native", "jump_threads.cpp"),
-                    os.path.join(CSRC, "jump.cpp"), os.path.join(CSRC, "mpview.cpp"),
-                    "-o", exe, "-l:libgmp.so.10", "-ldl"], check=True)
+def test_tables_keep_to_their_threads(threads, where, step, N):
     re, im = where if isinstance(where, tuple) else center(where)
-    out = subprocess.run([exe, re, im, step, "97", "131", str(N)], capture_output=True, text=True)
+    out = subprocess.run([threads, re, im, step, "97", "131", str(N)], capture_output=True,
+                         text=True)
     differ, beyond, started = out.stdout.split()
     assert differ == "0" and beyond == "0" and int(started) > 0, out.stdout
+
+
+# (center, step, N, grids of 2^17 - 1, 2^17, 499,999 and 500,000 samples with tables):
+# long start jumps; short ones; none, a center known to 15 digits far below them
+@pytest.mark.parametrize("where,step,N,tables", [
+    (25, "2e-28", 40000, "0111"),
+    (SEAHORSE, "2e-17", 50000, "0001"),
+    (SEAHORSE, "1e-28", 60000, "0000"),
+])
+def test_tables_only_where_they_pay(run, where, step, N, tables):
+    assert run("sizes", where, step, 333, 517, N, "center")[0] == tables
