@@ -352,15 +352,16 @@ __device__ __forceinline__ FF ff_norm2(FF x, FF y) {
 
 // The bailout test on Y = Z + delta (unscaled, float-float).  Returns true
 // when |Y|^2 > 2^20; clears `certified` when the error bound `yerr` on |Y|
-// reaches across 1024, or (kSmooth) when an escaped sample's exceeds |Y| / 16:
+// reaches across 1024, or (kSmooth) when an escaped sample's exceeds |Y| / 12:
 // the smoothing term moves by up to 0.21 of the relative error of |Y|.  Jumps leave
 // a bound nearer the error than a thousand steps' was, so that without this samples
 // of larger error are certified.  Largest difference from the FP64 path's smoothing
-// without jumps (no such test), and with |Y| / 8, / 16 and / 32: 1600x1200 at 2e-13
-// 4.8e-5, 5.0e-5, 2.8e-5, 1.6e-5; 1920x1080 at 1e-20 2.8e-5, 3.4e-5, 1.5e-5, 8.7e-6;
-// 960x540 at 1e-300 9.8e-5, 8.7e-5, 2.4e-5, 1.4e-5.  The frames: 1920x1080x16 at 1e-12
-// 166, 72, 74, 77 ms; 3840x2160 at 1e-300 89, 67.6, 68.1, 69.2, at 1e-330 247, 148,
-// 165, 185, at 1e-120 129, 90, 99, 110.
+// without jumps (no such test), and with |Y| / 8, / 10, / 12 and / 16: 1600x1200 at 2e-13
+// 4.8e-5, 5.0e-5, 4.8e-5, 4.2e-5, 2.8e-5; 1920x1080 at 2.5e-13 4.9e-5, 8.6e-5, 4.4e-5,
+// 3.2e-5, 3.2e-5, at 1e-20 2.8e-5, 3.4e-5, 2.0e-5, 1.9e-5, 1.5e-5; 3840x2160 at 1e-300
+// 1.2e-4, 8.8e-5, 6.4e-5, 4.5e-5, 4.3e-5.  The frames: 1920x1080x16 at 1e-12 167, 73.1,
+// 73.6, 72.8, 75.6 ms; 3840x2160 at 1e-300 90.8, 67.8, 67.6, 67.7, 68.8, at 1e-330 247,
+// 148, 153, 157, 165, at 1e-120 129, 90, 93, 95, 99.
 template <bool kSmooth>
 __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& certified,
                                                FF& r2) {
@@ -369,7 +370,7 @@ __device__ __forceinline__ bool fe_escape_test(FF yr, FF yi, float yerr, bool& c
   // | |Y| - 1024 | <= 2 yerr  <=>  | |Y|^2 - 2^20 | <= (2048 + 2 yerr) 2 yerr
   if (fabsf(d) <= up_fma(up_fma(2.0f, yerr, 2048.0f), up_mul(2.0f, yerr), up_mul(0x1p-40f, r2.h)))
     certified = false;
-  if (kSmooth && d > 0.0f && up_mul(256.0f * yerr, yerr) > r2.h) certified = false;
+  if (kSmooth && d > 0.0f && up_mul(144.0f * yerr, yerr) > r2.h) certified = false;
   return d > 0.0f;
 }
 
