@@ -619,23 +619,25 @@ void build_chain(const OrbitData& od, int s, double eps, JumpRec* out, int* stop
     double drop[B];
     dropped_by_square<B>(a, nb, rho[first], drop);
     for (int b = 1; b < nb; b++) drop[b] *= epow[b];
-    for (int i = std::min(first, lin); i <= lin; i++) {
-      double x = nb == 1 ? eps : 0.0;
-      for (int b = 1; b < nb; b++)
-        for (int c = nb - b; c < nb; c++) x += order[b][i] * order[c][i] * epow[b + c];
-      T[i] = x;
-    }
-    for (int i = 0; i < C; i++) {
-      if (!alive[i]) continue;
-      double h = T[std::min(i, lin)];
-      for (int b = 0; b < nb; b++) h += drop[b] * fall[b][i];
+    const int from = std::min(first, lin);
+    for (int i = from; i <= lin; i++) T[i] = nb == 1 ? eps : 0.0;
+    for (int b = 1; b < nb; b++)
+      for (int c = nb - b; c < nb; c++)
+        for (int i = from; i <= lin; i++) T[i] += order[b][i] * order[c][i] * epow[b + c];
+    for (int i = lin + 1; i < C; i++) T[i] = T[lin];
+    for (int b = 0; b < nb; b++)
+      for (int i = first; i < C; i++) T[i] += drop[b] * fall[b][i];
+    // (the balls that have ended among them: for whole vectors)
+    for (int i = first; i < C; i++) {
+      const double h = T[i];
       const double d = P[i] + E[i];
       R[i] = (2.0 * xm + 2.0 * d + R[i]) * R[i] + h;
       // as build_class, with eps's own terms
       Q[i] = (2.0 * xm + 2.0 * d + Q[i]) * Q[i] + h +
              0x1p-50 * (2.5 * 2.0 * xm * d + 9.5 * d * d) + 0x1p-48 * eps;
-      if (!(R[i] <= 0x1p-6 * P[i])) alive[i] = false;
     }
+    for (int i = first; i < C; i++)
+      if (!(R[i] <= 0x1p-6 * P[i])) alive[i] = false;
     if (nb == 1) continue;
     // Recentre (Shift) where the linear coefficient is the largest so far:
     // theta goes with its inverse, and after a near return of the orbit it is
@@ -751,13 +753,35 @@ void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, Jump
   if (starts.empty() || samples < kJumpFewSamples ||
       (few && (double)samples * starts[0].fire < kJumpStopSteps))
     return;
-  // the chain from a rebase, mostly the longest of these, then the start classes
+  // The chain from a rebase, mostly the longest of these, the start classes, and, on
+  // threads to spare, the chains that are likely to be wanted next: from past the
+  // smallest element of the orbit and past the smallest within a chain's reach.
   std::vector<int> stops(starts.size(), -1);
   int stop[kChains] = {-1, -1, -1};
-  const size_t first = chains ? 1 : 0;
+  std::vector<int> guess;
+  if (chains && threads > 2) {
+    for (const int reach : {kChainReach, od.xlen}) {
+      int at = -1;
+      double least = INFINITY;
+      for (int n = 64; n < std::min(reach, od.xlen); n++) {
+        const double m = od.xhi[n].x * od.xhi[n].x + od.xhi[n].y * od.xhi[n].y;
+        if (m < least) {
+          least = m;
+          at = n;
+        }
+      }
+      if (at >= 0 && std::find(guess.begin(), guess.end(), at + 1) == guess.end())
+        guess.push_back(at + 1);
+    }
+  }
+  std::vector<JumpRec> guessed(guess.size() * kChainClasses, none);
+  const size_t first = chains ? 1 + guess.size() : 0;
   run_on(threads, first + starts.size(), [&](size_t k) {
-    if (k < first)
+    int unused;
+    if (chains && k == 0)
       build_chain(od, 0, eps, &t.chain[0], &stop[0]);
+    else if (k < first)
+      build_chain(od, guess[k - 1], eps, &guessed[(k - 1) * kChainClasses], &unused);
     else
       build_class(od, starts[k - first], p, &t.start[(k - first) * kJumpSubs], &stops[k - first]);
   });
@@ -778,8 +802,17 @@ void build_jumps(const OrbitData& od, double eps_m, int eps_e, int threads, Jump
   };
   for (size_t k = 0; k < stops.size() && k < 2; k++) add(stops[k]);
   add(stop[0]);
-  run_on(threads, from.size() - 1, [&](size_t k) {
-    build_chain(od, from[k + 1], eps, &t.chain[(k + 1) * kChainClasses], &stop[k + 1]);
+  std::vector<size_t> rest;
+  for (size_t k = 1; k < from.size(); k++) {
+    const size_t g = std::find(guess.begin(), guess.end(), from[k]) - guess.begin();
+    if (g < guess.size())
+      std::copy_n(&guessed[g * kChainClasses], kChainClasses, &t.chain[k * kChainClasses]);
+    else
+      rest.push_back(k);
+  }
+  run_on(threads, rest.size(), [&](size_t i) {
+    const size_t k = rest[i];
+    build_chain(od, from[k], eps, &t.chain[k * kChainClasses], &stop[k]);
   });
   for (size_t k = 0; k < from.size(); k++) t.start_index[k] = from[k];
 }
