@@ -66,7 +66,8 @@ enum nm_path {
 enum nm_option {
   NM_OPT_TILE_W = 0,      /* sample order: tile width (default 16) */
   NM_OPT_TILE_H = 1,      /* tile height (default 16) */
-  NM_OPT_CHUNK = 2,       /* iterations between lane refills (default 32; 64 on the double loop) */
+  NM_OPT_CHUNK = 2,       /* iterations between lane refills, 1 and more (unset: 64 on the
+                             double loop, else 32; once set it holds for both) */
   NM_OPT_KEEP_SMOOTH64 = 3, /* 1: also keep the unrounded double smoothing */
   NM_OPT_THREADS = 4,     /* host threads for the probe search (0 = all) */
   NM_OPT_BLOCKS = 5,      /* persistent blocks (0 = fill the GPU) */

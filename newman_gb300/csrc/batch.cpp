@@ -17,7 +17,7 @@ using nmg::fail;
 struct nm_batch {
   int sc = 1;
   std::vector<nm_handle*> frames;
-  int tile_w = 16, tile_h = 16, chunk = 32, fe_chunk = 64;  // fe_chunk 64: the 240-frame zoom 1399 -> 1340 ms
+  int tile_w = 16, tile_h = 16, chunk = 0, fe_chunk = 64;  // fe_chunk 64: the 240-frame zoom 1399 -> 1340 ms
   bool use_graph = true;
   bool overlap = true;  // FP64 work inside the FE32 iteration pass
   int fp64_warps = 0;   // of 8 a block in that pass; 0: chosen from the batch
@@ -184,13 +184,15 @@ int build(nm_batch* b) {
   L.hw_ctl = ctl_at(w, kHwNext, kHwStats, L.hw.total);
   L.fp64_ctl = ctl_at(w, kFp64Next, kFp64Stats, L.fp64.total);
   L.fe_chunk = b->fe_chunk;
-  L.chunk = b->chunk;
+  L.chunk = nmg::chunk_steps(b->chunk, false);
+  L.hw_chunk = nmg::chunk_steps(b->chunk, true);
   L.overlap = b->overlap;
   L.fp64_warps = b->fp64_warps;
   L.overlap_ctl.rework = L.rework_ctl;
   L.overlap_ctl.fe_warps_done = w + kFeWarpsDone;
   L.overlap_ctl.timeouts = w + kFeStats + nmg::STAT_WAIT_TIMEOUTS;
-  L.overlap_ctl.chunk = b->chunk;
+  L.overlap_ctl.chunk = L.chunk;
+  L.overlap_ctl.hw_chunk = L.hw_chunk;
   L.reduce = b->d_reduce.p;
   L.nreduce = (int)red.size();
   L.reduce_total = red_total;

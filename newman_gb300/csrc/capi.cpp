@@ -868,6 +868,7 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
       o.fe_warps_done = h->d_scratch.p + kFeWarpsDone;
       o.timeouts = h->d_scratch.p + kStatsMain + nmg::STAT_WAIT_TIMEOUTS;
       o.chunk = h->fp64_chunk(false);
+      o.hw_chunk = h->fp64_chunk(true);
     }
     // No orbit entries staged unless asked for: a rebased sample leaves the first
     // entries by a jump, and the shared memory is better left to the L1 (3840x2160

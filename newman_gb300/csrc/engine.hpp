@@ -82,6 +82,7 @@ struct OverlapCtl {
   unsigned long long* fe_warps_done; // FP32 warps that finished their FP32 work
   unsigned long long* timeouts;      // waits that ran out (stats word)
   int chunk;                         // FP64 steps between refills
+  int hw_chunk;                      // the same for a batch's double-loop frames
 };
 constexpr unsigned int kListSentinel = 0xffffffffu;
 
@@ -122,7 +123,7 @@ struct BatchLaunch {
   bool overlap;             // FP64 work inside the FE32 iteration pass
   int fp64_warps;           // FP64 warps of 8 a block in that pass (0: by the batch)
   OverlapCtl overlap_ctl;   // its rework side (= rework_ctl) and counters
-  int fe_chunk, chunk;
+  int fe_chunk, chunk, hw_chunk;  // steps between refills: FE32, FP64, double loop
   const ReduceJob* reduce;  // [nreduce], device memory
   int nreduce;
   long long reduce_total;
@@ -132,6 +133,14 @@ cudaError_t launch_batch(const BatchLaunch& launch, cudaStream_t stream);
 // The FP64 render of the batch's rework list from its claim counter on (the
 // caller resets it), then the multisample reduce of every frame.
 cudaError_t launch_batch_rework(const BatchLaunch& launch, cudaStream_t stream);
+
+// Steps between refills of the FP64 and reference-exact kernels, as set (NM_OPT_CHUNK)
+// or 0: 64 on the double loop (1367x769x4 view at 3e-5: 20.4 -> 19.8 ms, a row of 640
+// samples 0.39 -> 0.38, eight frames of 640x360x4 from width 4 to 1e-9 in a batch 22.2 ->
+// 21.7), else 32.
+inline int chunk_steps(int set, bool double_loop) {
+  return set > 0 ? set : double_loop ? 64 : 32;
+}
 
 // Kernels launched by this library in this process (all handles; a graph
 // replay counts its kernel nodes).  note_launches adds n.

@@ -74,10 +74,7 @@ struct nm_handle {
   nmg::MPView view;
   int device = 0;
   int path = NM_PATH_REFERENCE;
-  // chunk 0: steps a chunk of the FP64 and reference-exact kernels, 64 on the double
-  // loop (1367x769x4 view at 3e-5: 20.4 -> 19.8 ms, a row of 640 samples 0.39 ->
-  // 0.38), else 32
-  int fp64_chunk(bool double_loop) const { return chunk > 0 ? chunk : double_loop ? 64 : 32; }
+  int fp64_chunk(bool double_loop) const { return nmg::chunk_steps(chunk, double_loop); }
   // renorm 0: 64 steps a chunk (with 32, 64 and 128: 1920x1080x16 at width 1e-12 89.4,
   // 85.7, 84.7 ms; 3840x2160 at 1e-300 66.0, 63.0, 62.4; 2x2 samples at 1e-412 1,086 each)
   int tile_w = 16, tile_h = 16, chunk = 0, blocks = 0, threads = 0, renorm = 0;

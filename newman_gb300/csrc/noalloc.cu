@@ -106,7 +106,8 @@ extern "C" int nm_render_fe32_noalloc(nm_handle* h, nm_escape_value* out, void* 
   ctl.rework_n = s ? s->words + kReworkCount : nullptr;
   if (e == cudaSuccess && kind == nmg::KERNEL_HW) {
     e = nmg::launch_render(nmg::KERNEL_HW, v, ctl, st,
-                           nmg::persistent_blocks(nmg::KERNEL_HW, device), 32);
+                           nmg::persistent_blocks(nmg::KERNEL_HW, device),
+                           nmg::chunk_steps(0, true));
   } else if (e == cudaSuccess) {
     e = nmg::launch_render(nmg::KERNEL_FE32, v, ctl, st,
                            nmg::persistent_blocks(nmg::KERNEL_FE32, device), 16);

@@ -201,7 +201,7 @@ __device__ __noinline__ void batch_fp64_side(const BatchGroup& fe, const BatchGr
                                              const RenderCtl& hw_ctl, const OverlapCtl& o,
                                              unsigned long long producers,
                                              SamplePool<Fp64AnyJob::State>* pool) {
-  if (hw.n > 0) sample_loop<HwJob>(Frames{hw}, hw_ctl, o.chunk);
+  if (hw.n > 0) sample_loop<HwJob>(Frames{hw}, hw_ctl, o.hw_chunk);
   drain_loop<Fp64AnyJob>(Frames{fe}, o.rework, o.fe_warps_done, producers, o.timeouts, o.chunk,
                          pool);
 }
@@ -319,7 +319,7 @@ cudaError_t launch_batch(const BatchLaunch& L, cudaStream_t s) {
   if (L.hw.n > 0 && L.hw.total > 0)
     batch_list_kernel<HwJob>
         <<<blocks_of((const void*)batch_list_kernel<HwJob>, kPersistentThreads, dev),
-           kPersistentThreads, 0, s>>>(L.hw, L.hw_ctl, L.chunk);
+           kPersistentThreads, 0, s>>>(L.hw, L.hw_ctl, L.hw_chunk);
   if (L.fp64.n > 0 && L.fp64.total > 0) note_launches(1);
   if (L.fp64.n > 0 && L.fp64.total > 0)
     batch_list_kernel<Delta64Job>
