@@ -872,9 +872,9 @@ int nm_render_rows(nm_handle* h, int r0, int r1, void* stream_arg) {
     }
     // No orbit entries staged unless asked for: a rebased sample leaves the first
     // entries by a jump, and the shared memory is better left to the L1 (3840x2160
-    // at width 1e-300 with 0, 512 and 1024 entries 63.0, 64.7, 64.8 ms; at 1e-330
-    // 161, 166, 165; 2x2 samples at 1e-412 1,086, 1,110, 1,127; the 1920x1080x16 view
-    // at 1e-12 with 0 and 1024 84.5, 86.2).
+    // at width 1e-300 with 0, 512 and 1,000 entries 68.5, 69.7, 69.4 ms; at 1e-330
+    // 157, 160, 159; 2x2 samples at 1e-412 1,160, 1,177, 1,192; the 1920x1080x16 view
+    // at 1e-12 within its spread).
     const int stage = h->z_stage >= 0 ? h->z_stage : 0;
     NM_CUDA(nmg::launch_fe32_passes(v, b, ctl, s, h->device, h->blocks, chunk, h->ev[3],
                                     h->ev[4], h->fe_overlap ? &o : nullptr, stage,

@@ -5,8 +5,8 @@
 //
 // delta, eps and the reference orbit Z are float-float pairs (two FP32 words)
 // and, while |delta| < 2^-60, delta and eps share one int exponent E per
-// sample (delta = mantissa * 2^E), renormalised at the end of every chunk of
-// steps and whenever the mantissa passes 2^60.
+// sample (delta = mantissa * 2^E), renormalised every NM_OPT_RENORM steps of the
+// sample, in whatever pieces they are made, and whenever the mantissa passes 2^60.
 //
 // Certification.  Alongside delta the iteration propagates a bound on the
 // absolute error of delta against exact arithmetic from the same start,

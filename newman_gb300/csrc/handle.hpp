@@ -75,8 +75,9 @@ struct nm_handle {
   int device = 0;
   int path = NM_PATH_REFERENCE;
   int fp64_chunk(bool double_loop) const { return nmg::chunk_steps(chunk, double_loop); }
-  // renorm 0: 64 steps a chunk (with 32, 64 and 128: 1920x1080x16 at width 1e-12 89.4,
-  // 85.7, 84.7 ms; 3840x2160 at 1e-300 66.0, 63.0, 62.4; 2x2 samples at 1e-412 1,086 each)
+  // renorm 0: 64 steps a round and between renormalisations (with 16, 32, 64 and 128:
+  // 1920x1080x16 at width 1e-12 87.2, 76.2, 69.1, 69.2 ms; 3840x2160 at 1e-300 74.0,
+  // 68.8, 65.1, 65.1, at 1e-330 149.3, 148.8, 148.8, 148.4)
   int tile_w = 16, tile_h = 16, chunk = 0, blocks = 0, threads = 0, renorm = 0;
   bool keep_smooth64 = false;
   cudaStream_t stream = nullptr;

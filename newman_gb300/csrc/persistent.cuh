@@ -197,8 +197,8 @@ __device__ __forceinline__ bool pool_exchange(SamplePool<typename Job::State>* p
 // A warp takes new samples once Job::kRefill lanes are empty (or all work has to
 // start): the series front in FP64 costs the warp the same for one lane as for
 // four, some 100 FP64 instructions (FE32 rework of the 1920x1080x16 view at
-// 1e-12 with 1, 4 and 8 lanes: 117, 86, 86 ms for the frame; the FP64 path there,
-// 961x541x4: 84, 81, 80 ms).  A double-loop start is cheap and its samples can be
+// 1e-12 with 1, 4 and 8 lanes: 119, 73-77, 70 ms for the frame; the FP64 path there,
+// 961x541x4: 84, 80, 80 ms).  A double-loop start is cheap and its samples can be
 // short: one lane (640x480 view of width 3: 0.71, 0.73, 0.77 ms).  The
 // reference-exact path gains nothing either way (one lane).
 template <class Job, class Src>

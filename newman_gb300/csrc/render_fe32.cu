@@ -12,11 +12,11 @@
 //                       and appends it to a work list, or finishes it
 //                       (cardioid, escape before the skip point).
 //     fe_overlap_kernel persistent and warp-refilled over the work list: six
-//                       warps a block run the FP32 delta iteration and the
-//                       smoothing term, appending every sample they cannot
-//                       certify to the rework list, which the other two warps
-//                       render in FP64 meanwhile (fe_iter_kernel: the FP32
-//                       warps alone, the rework after the pass).
+//                       or five warps a block run the FP32 delta iteration,
+//                       the jumps and the smoothing term, appending every sample
+//                       they cannot certify to the rework list, which the other
+//                       two or three render in FP64 meanwhile (fe_iter_kernel:
+//                       the FP32 warps alone, the rework after the pass).
 //   followed by the plain FP64 kernel over what is left of the rework list.
 //   FP64 runs only in converged warps: GB300 issues FP64 at about 1/75 of the
 //   FP32 rate, and a warp instruction costs the FP64 pipe the same whatever
@@ -211,18 +211,17 @@ __global__ void __launch_bounds__(kPersistentThreads) fe_iter_kernel(DeviceView 
 // FP64 code under this kernel's 64-register cap spills; a warp joining it
 // made a 3840x2160 (2x2) view of width 1e-413 5 % slower and helped nowhere).
 // Capped at 64 registers so that 4 blocks fit on an SM (3 blocks at 80: the
-// 1920x1080x16 view of width 1e-12 86 ms either way).  Two FP64 warps a block there:
-// three or four only spread the same FP64 work over more, emptier warps (85, 90, 98
-// ms; with the rework after the pass 112).  Floatexp views and those of many
-// iterations rework more samples, for longer, and take three
-// (2 -> 3 warps: 3840x2160 at 1e-40, N 1e6 114 -> 97 ms, at 1e-120 105 -> 90, at 1e-300
-// 64 -> 63, at 1e-330 184 -> 162, 2x2 samples at 1e-412 1,258 -> 1,086; at 1e-500, where
-// the FP32 side is the longer one, 233 -> 241); four: 69, 163, 1,183, 270 on the
-// last four.  What decides is the share of reworked samples, known only afterwards:
-// from 4 % on three are faster (2x2 at 1e-20, N 50,000 182 -> 157), near 2 % two
-// (1e-60 30.5 -> 28.4 ms with N 100,000 or more).  A sixth FP32 warp that changed
-// sides on a backlog of 32 entries a block came within 2 % of the better of the two
-// on the deep views and gave 88 ms on the 1e-12 one.
+// 1920x1080x16 view of width 1e-12 86 ms either way).  Two FP64 warps a block there
+// (2, 3 and 4: 73, 74, 84 ms; with the rework after the pass 104).  Floatexp views and
+// those of many iterations rework more samples, for longer, and take three (2, 3 and
+// 4 warps: 3840x2160 at 1e-40, N 1e6 117, 101, 101 ms, at 1e-120 111, 95, 94, at 1e-300
+// 70, 67, 73, at 1e-330 175, 157, 157, 2x2 samples at 1e-412 1,367, 1,160, 1,218, at
+// 1e-500, where the FP32 side is the longer one, 252, 249, 278).  What decides is the
+// share of reworked samples, known only afterwards, and a rule by the view misses some:
+// 3840x2160 at 1e-20, N 50,000 (5.7 % reworked) takes two and 76 ms, 67 with three; at
+// 1e-60 (2.4 %) three and 31 ms, 29 with two.  A sixth FP32 warp that
+// changed sides on a backlog of 32 entries a block came within 2 % of the better of
+// the two on the deep views and was 4 % slower on the 1e-12 one.
 int fp64_warps_for(const DeviceView& v) { return (v.sa_fe || v.N > 200000) ? 3 : 2; }
 
 // The FP64 side, out of line: its register pressure (the FP64 series front)
